@@ -57,7 +57,9 @@ OTHER_WORKLOADS = ("batch64", "serve", "makeindex", "couple256")
 # (FP64 13-row tiles, FP32 29-row tiles): not measured in the run that
 # reports them.
 SWEEP_DRAM_BYTES_PER_CELL = {"fp64": 67.8, "fp32-mixed": 35.5}
-SWEEP_KERNELS = ("hsmac_rw", "hsmac_fused")
+SWEEP_KERNELS = ("pot_sweep", "hsmac_rw", "hsmac_fused")
+# the same of pot_sweep, which does three sweeps a launch (512^3 captures)
+POT_DRAM_BYTES_PER_CELL = {"fp64": 39.0, "fp32-mixed": 18.6}
 # FP64 operations per interior cell of one rhs!+update! launch (k_rhs, both
 # stages alike): smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on
 # of an ncu capture of k_rhs at 128^3: 484.4 M adds + 471.9 M multiplies, no
@@ -179,20 +181,23 @@ def kernel_table(tot, n, h, T, particles_per_launch, peak):
 
 
 def sweep_roofline(tot, n3, precision, peak, peak_kind):
-    """HBM roofline of the dominant kernel, the fused red-black sweep: 8T bytes
-    per interior cell (U, V, W, P read and written once) over its average
-    CUDA-event launch time."""
+    """HBM roofline of the dominant kernel over its average CUDA-event launch
+    time: pot_sweep, three red-black sweeps of the potential (3T bytes per
+    interior cell: Phi and the right-hand side read, Phi written), or the
+    element-wise sweep (8T: U, V, W, P read and written once)."""
     k = max(SWEEP_KERNELS, key=lambda s: tot.get(s, (0.0, 0))[0])
     ms, cnt = tot.get(k, (0.0, 0))
     T = elem_bytes(precision)
-    alg = 8 * T * n3
+    pot = k == "pot_sweep"
+    alg = (3 if pot else 8) * T * n3
+    per_cell = (POT_DRAM_BYTES_PER_CELL if pot else SWEEP_DRAM_BYTES_PER_CELL)[precision]
     avg = ms / max(cnt, 1)
     ach = alg / (avg / 1e3) / 1e9 if cnt else None
     return {"kernel": k, "bound": "hbm", "achieved": ach, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
-            "frac": (ach / peak) if ach else None, "traffic": SWEEP_DRAM_BYTES_PER_CELL[precision] * n3,
+            "frac": (ach / peak) if ach else None, "traffic": per_cell * n3,
             "traffic_source": "not measured in this run: ncu dram__bytes_read.sum + dram__bytes_write.sum per "
-                              f"interior cell of a 256^3 capture of the same kernel (a D2 sweep, "
-                              f"{SWEEP_DRAM_BYTES_PER_CELL[precision]} B), times n^3",
+                              f"interior cell of a {'512^3' if pot else '256^3'} capture of the same kernel "
+                              f"({per_cell} B), times n^3",
             "alg_bytes_per_launch": alg, "avg_launch_ms": avg, "launches_profiled": cnt}
 
 
@@ -669,11 +674,14 @@ def run_serve(args):
 def kernel_bytes(n, h, T, particles_per_launch):
     """Algorithmic DRAM bytes per launch of the step's kernels (n^3 grid, halo
     h, T-byte field elements):
+    - pot_sweep: Phi and its right-hand side read, Phi written, 3T x n^3 (three
+      sweeps); pot_setup: U, V, W read, the two written, 5T; pot_apply: Phi, U,
+      V, W, P read, the last four written, 9T;
     - hsmac_rw: U, V, W, P read and written once per cell, 8T x n^3;
     - hsmac_faces: the same per cell of the six face slabs of the first
       time-blocked sweep's box -1..n+3 around the core 2..n;
-    - synchalo: the couple's fill (radius h, all 26 directions, U, V, W): one
-      read and one write per halo cell;
+    - synchalo: a fill of radius h in all 26 directions of U, V, W: one read and
+      one write per halo cell;
     - rhs_update: stage 1 reads U, V, W, P, writes U2, V2, W2 (7T); stage 2
       also reads U2, V2, W2 (10T): the mean, 8.5T x n^3;
     - particles: 13 FP64 properties read or written a particle, the mean of the
@@ -682,7 +690,7 @@ def kernel_bytes(n, h, T, particles_per_launch):
     n3 = float(n) ** 3
     slab = float(n + 5) ** 3 - float(n - 1) ** 3
     halo = float(n + 2 * h) ** 3 - n3
-    return {"hsmac_rw": 8 * T * n3, "hsmac_faces": 8 * T * slab, "synchalo": 3 * 2 * T * halo,
+    return {"pot_sweep": 3 * T * n3, "pot_setup": 5 * T * n3, "pot_apply": 9 * T * n3, "hsmac_rw": 8 * T * n3, "hsmac_faces": 8 * T * slab, "synchalo": 3 * 2 * T * halo,
             "rhs_update": 8.5 * T * n3, "particles": 128.0 * particles_per_launch, "cfl_max": 3 * T * n3}
 
 

@@ -105,6 +105,11 @@ struct Ctx {
   // 2 makes the sweep's TMA plane barriers expect 16 bytes more than its
   // copies deliver; either wait then runs out at its bound.  0 in production.
   int debug_wait;
+  // couple in potential form (lcs_potential.cuh)
+  int pot_cur;      // which spare buffer holds the group's input potential
+  int pot_pending;  // the last group's jumps are not yet in the right-hand side
+  int pot_redo;     // sweeps of the group to run again (the exit lay inside it), 0: none
+  double pot_floor; // mean square divergence of the FP32 velocity's rounding (0 in FP64)
 };
 
 // ---- stencil primitives (src/diff.jl:1-39), same evaluation order --------

@@ -26,6 +26,7 @@
 #include "lcs_kernels.cuh"
 #include "lcs_tma.cuh"
 #include "lcs_hsmac_rw.cuh"
+#include "lcs_potential.cuh"
 #include "lcs_makeindex.cuh"
 #include "lcs_pstat.cuh"
 
@@ -180,6 +181,7 @@ class Engine : public EngineBase {
   const std::vector<Engine<T>*>* grp = nullptr;
   int tuning_gen = 0;            // bumped by set_tuning (a group's graph is rebuilt)
   GroupPtrs<T> grp_ptrs{};       // per member Ctx, P, partials (set by the group)
+  PotGroup<T> pot_ptrs{}, grp_pot{};  // the same for the potential form: this handle alone, its group
   int face_group_per_sm = 0;     // co-resident blocks per SM of k_hsmac_faces_group
   // scratch of the particle statistics (grown on demand)
   char* pbuf = nullptr;
@@ -311,8 +313,127 @@ class Engine : public EngineBase {
       return fail(LCS_EINVAL, "a field of 2^32 or more elements");
     if (use_rw) LCS_TRY(init_tma());
     LCS_TRY(init_faces());
+    LCS_TRY(init_pot());
     LCS_CUDA(cudaStreamSynchronize(stream));
     return LCS_OK;
+  }
+
+  // ------------------------------------------------------- potential form
+  // The time-blocked couple in potential form (lcs_potential.cuh) serves
+  // red-black-fast.  LCS_B200_FUSED_SWEEP = rw or plain, or a variable that
+  // shapes those sweeps (LCS_B200_RW, _FACES, _ZCHUNK), selects the
+  // element-wise sweeps, and so does the test hook of their device waits.
+  // FP64 grids of up to 40^3 cells keep them too: there they give the in-place
+  // order's bits, and a step is a few milliseconds either way.
+  bool pot_ok = false;
+  int debug_kind = 0;
+  bool use_pot() const { return pot_ok && debug_kind == 0; }
+    // tile of the sweep: FP64 8 warps of 4 rows.  FP32 12 warps of 4 rows on
+  // grids of more than 256^3 cells, where fewer redundant rows count, and 16 of
+  // 2 rows up to there, where a plane's latency does.
+  static constexpr int kPotR = 4, kPotW = sizeof(T) == 8 ? 8 : 12, kPotRS = sizeof(T) == 8 ? 4 : 2, kPotWS = sizeof(T) == 8 ? 8 : 16;
+  bool pot_small = true;
+  using PotT = PotTile<T, kPotW, kPotR>;
+  using PotS = PotTile<T, kPotWS, kPotRS>;
+  static constexpr size_t kSlabSmem = (size_t)10 * 1024 * sizeof(T);
+  int init_pot() {
+    const char* sweep = std::getenv("LCS_B200_FUSED_SWEEP");
+    const std::string sw = sweep ? std::string(sweep) : std::string();
+    const bool shaped = std::getenv("LCS_B200_RW") || std::getenv("LCS_B200_FACES") || std::getenv("LCS_B200_ZCHUNK");
+    const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2];
+    const PotScratch ps = pot_scratch(g.n, (int)sizeof(T));
+    pot_ok = cfg.coloring == LCS_COLORING_RED_BLACK_FAST && cfg.time_blocking && g.n[0] >= 8 && g.n[1] >= 8 &&
+             g.n[2] >= 8 && g.elems < INT32_MAX &&
+             (int64_t)ps.pz * (g.n[2] + 5) <= g.elems &&
+             (size_t)ps.total * sizeof(T) <= (size_t)plan.stage_elems * sizeof(double) &&
+             (sw == "potential" || (sw.empty() && !shaped && (sizeof(T) == 4 || cells > 40 * 40 * 40)));
+    if (!pot_ok) return LCS_OK;
+    pot_small = cells <= 256 * 256 * 256;
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotW, kPotR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)PotT::bytes));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotWS, kPotRS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)PotS::bytes));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
+    pot_ptrs.ctx[0] = dctx;
+    pot_ptrs.P[0] = P;
+    pot_ptrs.scratch[0] = (T*)stage;
+    pot_ptrs.partials[0] = partials;
+    return LCS_OK;
+  }
+  PotGeom pot_geom() const {
+    PotGeom pg;
+    memset(&pg, 0, sizeof pg);
+    pg.s = pot_scratch(g.n, (int)sizeof(T));
+    pg.overlap = cfg.overlap ? 1 : 0;
+    const int ty = pot_small ? PotS::TY : PotT::TY;
+    pg.gx = (g.n[0] + 1 + PotT::TX - 1) / PotT::TX;
+    pg.gy = (g.n[1] + 1 + ty - 1) / ty;
+    // A CTA takes one of nc z chunks of a tile column; its time is its planes
+    // and the 12 more that fill and drain the six half sweeps.
+    const int cols = pg.gx * pg.gy, nu = (g.n[2] + 2) / 2, slots = share_slots(num_sms);
+    double best = 1e300;
+    const int cu = zchunk_force > 0 ? (zchunk_force + 1) / 2 : 0;  // units of two planes of a forced chunk
+    for (int nc = std::max(cu > 0 ? (nu + cu - 1) / cu : 1, (2 * nu + kPotMaxChunk - 1) / kPotMaxChunk); nc <= nu; nc++) {
+      const double cost = std::ceil((double)cols * nc / slots) * (2.0 * ((nu + nc - 1) / nc) + 12.0);
+      if (cost < best - 1e-9) {
+        best = cost;
+        pg.nc = nc;
+        pg.nseg = cols * nc;
+      }
+      if (cu > 0 || (int64_t)cols * nc > 64 * (int64_t)slots) break;
+    }
+    pg.slab_part = 3 * pg.nseg;
+    if (cfg.overlap)
+      for (int a = 0; a < 3; a++) pg.nslab += slab_tiles(a).x * slab_tiles(a).y;
+    pg.cx = hc.dxi * hc.dxi;
+    pg.cy = hc.dyi * hc.dyi;
+    pg.cz = hc.dzi * hc.dzi;
+    pg.k0 = 2.0 * (pg.cx + pg.cy + pg.cz);
+    pg.wd = -hc.omega * hc.dl;
+    pg.dxi = hc.dxi;
+    pg.dyi = hc.dyi;
+    pg.dzi = hc.dzi;
+    return pg;
+  }
+  dim3 slab_tiles(int a) const {  // tiles of the slabs normal to axis a
+    const int lu = a == 0 ? g.n[1] - 1 : g.n[0] + 5, lv = a == 2 ? g.n[1] + 5 : g.n[2] - 1;
+    return dim3((lu + kPotSlab - 1) / kPotSlab, (lv + kPotSlab - 1) / kPotSlab, 1);
+  }
+  const PotGroup<T>& pot_args() const { return grp ? grp_pot : pot_ptrs; }
+  int pot_members() const { return grp ? (int)grp->size() : 1; }
+  int pot_setup(int set) {
+    const PotGeom pg = pot_geom();
+    const int64_t half = (int64_t)g.n[0] / 2 * g.n[1] * g.n[2];
+    return launch("pot_setup", k_pot_setup<T>, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
+  }
+  int pot_apply(int set) {
+    const PotGeom pg = pot_geom();
+    const int64_t half = (int64_t)g.n[0] / 2 * g.n[1] * g.n[2];
+    return launch("pot_apply", k_pot_apply<T>, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
+  }
+  // one group of three sweeps
+  int pot_group() {
+    const PotGeom pg = pot_geom();
+    const int M = pot_members();
+    if (3 * (int64_t)pg.nseg + pg.nslab > plan.partials_cap) return fail(LCS_EINVAL, "grid too large for the partials buffer");
+    const int64_t faces = (int64_t)g.n[0] * g.n[1] + (int64_t)g.n[0] * g.n[2] + (int64_t)g.n[1] * g.n[2];
+    LCS_TRY(launch("pot_jump", k_pot_jump<T>, dim3(blocks_for(faces, 256), M), dim3(256), 0, pot_args(), pg));
+    if (cfg.overlap) {
+      int part = pg.slab_part;
+      dim3 t = slab_tiles(2);
+      LCS_TRY(launch("pot_slab", k_pot_slab<T, 2>, dim3(t.x, t.y, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg, part));
+      part += t.x * t.y;
+      t = slab_tiles(1);
+      LCS_TRY(launch("pot_slab", k_pot_slab<T, 1>, dim3(t.x, t.y, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg, part));
+      part += t.x * t.y;
+      t = slab_tiles(0);
+      LCS_TRY(launch("pot_slab", k_pot_slab<T, 0>, dim3(t.x, t.y, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg, part));
+    }
+    if (pot_small)
+      return launch("pot_sweep", k_pot_sweep<T, kPotWS, kPotRS>, dim3(pg.nseg, M), dim3(PotS::NT), PotS::bytes, pot_args(), pg, hc, 1);
+    return launch("pot_sweep", k_pot_sweep<T, kPotW, kPotR>, dim3(pg.nseg, M), dim3(PotT::NT), PotT::bytes, pot_args(), pg, hc, 1);
   }
 
   // ---------------------------------------------------------- tensor maps
@@ -801,6 +922,7 @@ class Engine : public EngineBase {
   }
   // One iteration of the reference's `while itr < itrmax` loop.
   int couple_group(int set) {
+    if (use_pot()) return pot_group();
     const int n0 = g.n[0], h = g.h;
     (void)n0;
     const Box full = cube(g, 1 - h, h);
@@ -843,12 +965,14 @@ class Engine : public EngineBase {
   int couple_direct(int stage) {
     const int set = stage == 1 ? kSetUs2 : kSetUs;  // Us_couple (couple.jl:1-2)
     LCS_TRY(launch("couple_reset", k_couple_reset, dim3(1), dim3(1), 0, dctx, cfg.itrmax));
+    if (use_pot()) LCS_TRY(pot_setup(set));
     int itr = 0;
     const int spg = sweeps_per_group();
     // the device advances itr by one per sweep until it exits; the group
     // count is bounded so the host loop ends even if that ever failed
     const int max_groups = max_loop_groups();
-    for (int grp = 0; itr < cfg.itrmax; grp++) {
+    bool again = false;  // the exit lay inside a potential-form group, which runs again up to it
+    for (int grp = 0; itr < cfg.itrmax || again; grp++) {
       if (grp >= max_groups) return fail(LCS_ETIMEDOUT, "HSMAC loop did not advance");
       LCS_TRY(couple_group(set));
       const int last_itr_in_group = itr + spg - 1;
@@ -858,10 +982,12 @@ class Engine : public EngineBase {
         if (hctx->nonfinite) return fail(LCS_ENONFINITE, "HSMAC residual is not finite");
         if (hctx->cs.done) break;
         itr = hctx->cs.itr;
+        again = use_pot() && hctx->pot_redo != 0;
       } else {
         itr += spg;
       }
     }
+    if (use_pot()) LCS_TRY(pot_apply(set));
     return launch("couple_log", k_couple_log, dim3(1), dim3(1), 0, dctx, stage);
   }
 
@@ -938,6 +1064,7 @@ class Engine : public EngineBase {
   int couple_graph_nodes(int stage) {
     const int set = stage == 1 ? kSetUs2 : kSetUs;
     LCS_TRY(launch("couple_reset", k_couple_reset, dim3(1), dim3(1), 0, dctx, cfg.itrmax));
+    if (use_pot()) LCS_TRY(pot_setup(set));
     cudaStreamCaptureStatus st;
     cudaGraph_t graph;
     const cudaGraphNode_t* deps = nullptr;
@@ -969,6 +1096,7 @@ class Engine : public EngineBase {
     if (rc2 != LCS_OK) return rc2;
     if (e != cudaSuccess) return fail(LCS_ECUDA, "capture of the couple loop: %s", cudaGetErrorString(e));
     LCS_CUDA(cudaStreamUpdateCaptureDependencies(stream, &node, 1, cudaStreamSetCaptureDependencies));
+    if (use_pot()) LCS_TRY(pot_apply(set));
     return launch("couple_log", k_couple_log, dim3(1), dim3(1), 0, dctx, stage);
   }
 
@@ -1491,6 +1619,11 @@ class Engine : public EngineBase {
     if (kind < 0 || kind > 2) return fail(LCS_EINVAL, "debug wait kind must be 0, 1 or 2");
     if (async_pending) return fail(LCS_ESTATE, "asynchronous steps are in flight on this handle");
     LCS_TRY(launch("set_debug_wait", k_set_debug_wait, dim3(1), dim3(1), 0, dctx, kind));
+    if (pot_ok && (kind != 0) != (debug_kind != 0)) {  // the waits are those of the element-wise sweeps
+      tuning_gen++;
+      drop_graphs();
+    }
+    debug_kind = kind;
     LCS_CUDA(cudaStreamSynchronize(stream));
     return LCS_OK;
   }
@@ -1972,6 +2105,12 @@ struct EngineGroup : GroupBase {
     Engine<T>* L = mem[0];
     const int set = stage == 1 ? kSetUs2 : kSetUs;
     LCS_GTRY(L, member_op(2, stage, "couple_reset"));
+    if (L->use_pot()) {
+      L->grp = &mem;
+      const int rs = L->pot_setup(set);
+      L->grp = nullptr;
+      LCS_GTRY(L, rs);
+    }
     cudaStream_t s = L->stream;
     cudaStreamCaptureStatus st;
     cudaGraph_t gr;
@@ -2009,6 +2148,12 @@ struct EngineGroup : GroupBase {
     cudaStreamDestroy(side);
     if (rc2 != LCS_OK) return rc2;
     LCS_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
+    if (L->use_pot()) {
+      L->grp = &mem;
+      const int ra = L->pot_apply(set);
+      L->grp = nullptr;
+      LCS_GTRY(L, ra);
+    }
     LCS_GTRY(L, member_op(3, stage, "couple_log"));
     return LCS_OK;
   }
@@ -2170,6 +2315,7 @@ int Engine<T>::group_create(EngineBase* const* members, int m, GroupBase** out) 
                       a.omega == b.omega && a.epsp == b.epsp && a.itrmin == b.itrmin && a.itrmax == b.itrmax;
     if (!same) return fail(LCS_EINVAL, "group members differ in shape or HSMAC settings");
     if (!e->use_rw) return fail(LCS_EINVAL, "group members need the row-warp sweep");
+    if (e->use_pot() != L->use_pot()) return fail(LCS_EINVAL, "group members differ in the form of the couple");
     if (e->rw_variant != L->rw_variant || e->zchunk_force != L->zchunk_force || e->sm_share != L->sm_share)
       return fail(LCS_EINVAL, "group members differ in launch shapes");
     if (e->async_pending) return fail(LCS_ESTATE, "asynchronous steps are in flight on a member");
@@ -2180,6 +2326,10 @@ int Engine<T>::group_create(EngineBase* const* members, int m, GroupBase** out) 
     L->grp_ptrs.ctx[q] = gp->mem[q]->dctx;
     L->grp_ptrs.P[q] = gp->mem[q]->P;
     L->grp_ptrs.partials[q] = gp->mem[q]->partials;
+    L->grp_pot.ctx[q] = gp->mem[q]->dctx;
+    L->grp_pot.P[q] = gp->mem[q]->P;
+    L->grp_pot.scratch[q] = (T*)gp->mem[q]->stage;
+    L->grp_pot.partials[q] = gp->mem[q]->partials;
   }
   gp->per_step.assign(m, 0);
   gp->gens.assign(m, -1);
