@@ -353,9 +353,7 @@ class Engine : public EngineBase {
                                   (int)PotT::bytes));
     LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotWS, kPotRS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)PotS::bytes));
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
     pot_ptrs.ctx[0] = dctx;
     pot_ptrs.P[0] = P;
     pot_ptrs.scratch[0] = (T*)stage;
@@ -386,7 +384,11 @@ class Engine : public EngineBase {
     }
     pg.slab_part = 3 * pg.nseg;
     if (cfg.overlap)
-      for (int a = 0; a < 3; a++) pg.nslab += slab_tiles(a).x * slab_tiles(a).y;
+      for (int a = 2; a >= 0; a--) {
+        pg.slab0[a] = pg.nslab;
+        const int lu = a == 0 ? g.n[1] - 1 : g.n[0] + 5, lv = a == 2 ? g.n[1] + 5 : g.n[2] - 1;
+        pg.nslab += ((lu + kPotSlab - 1) / kPotSlab) * ((lv + kPotSlab - 1) / kPotSlab);
+      }
     pg.cx = hc.dxi * hc.dxi;
     pg.cy = hc.dyi * hc.dyi;
     pg.cz = hc.dzi * hc.dzi;
@@ -397,11 +399,10 @@ class Engine : public EngineBase {
     pg.dzi = hc.dzi;
     return pg;
   }
-  dim3 slab_tiles(int a) const {  // tiles of the slabs normal to axis a
-    const int lu = a == 0 ? g.n[1] - 1 : g.n[0] + 5, lv = a == 2 ? g.n[1] + 5 : g.n[2] - 1;
-    return dim3((lu + kPotSlab - 1) / kPotSlab, (lv + kPotSlab - 1) / kPotSlab, 1);
-  }
   const PotGroup<T>& pot_args() const { return grp ? grp_pot : pot_ptrs; }
+  // groups in the body of a couple's loop in a step graph (those after the exit
+  // return at once)
+  int pot_unroll() const { return cfg.itrmax >= 24 ? 4 : 1; }
   int pot_members() const { return grp ? (int)grp->size() : 1; }
   int pot_setup(int set) {
     const PotGeom pg = pot_geom();
@@ -414,26 +415,17 @@ class Engine : public EngineBase {
     return launch("pot_apply", k_pot_apply<T>, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
   }
   // one group of three sweeps
-  int pot_group() {
+  int pot_group(const PotLoop& loop) {
     const PotGeom pg = pot_geom();
     const int M = pot_members();
     if (3 * (int64_t)pg.nseg + pg.nslab > plan.partials_cap) return fail(LCS_EINVAL, "grid too large for the partials buffer");
     const int64_t faces = (int64_t)g.n[0] * g.n[1] + (int64_t)g.n[0] * g.n[2] + (int64_t)g.n[1] * g.n[2];
     LCS_TRY(launch("pot_jump", k_pot_jump<T>, dim3(blocks_for(faces, 256), M), dim3(256), 0, pot_args(), pg));
-    if (cfg.overlap) {
-      int part = pg.slab_part;
-      dim3 t = slab_tiles(2);
-      LCS_TRY(launch("pot_slab", k_pot_slab<T, 2>, dim3(t.x, t.y, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg, part));
-      part += t.x * t.y;
-      t = slab_tiles(1);
-      LCS_TRY(launch("pot_slab", k_pot_slab<T, 1>, dim3(t.x, t.y, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg, part));
-      part += t.x * t.y;
-      t = slab_tiles(0);
-      LCS_TRY(launch("pot_slab", k_pot_slab<T, 0>, dim3(t.x, t.y, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg, part));
-    }
+    if (cfg.overlap)
+      LCS_TRY(launch("pot_slab", k_pot_slab<T>, dim3(pg.nslab, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg));
     if (pot_small)
-      return launch("pot_sweep", k_pot_sweep<T, kPotWS, kPotRS>, dim3(pg.nseg, M), dim3(PotS::NT), PotS::bytes, pot_args(), pg, hc, 1);
-    return launch("pot_sweep", k_pot_sweep<T, kPotW, kPotR>, dim3(pg.nseg, M), dim3(PotT::NT), PotT::bytes, pot_args(), pg, hc, 1);
+      return launch("pot_sweep", k_pot_sweep<T, kPotWS, kPotRS>, dim3(pg.nseg, M), dim3(PotS::NT), PotS::bytes, pot_args(), pg, hc, loop);
+    return launch("pot_sweep", k_pot_sweep<T, kPotW, kPotR>, dim3(pg.nseg, M), dim3(PotT::NT), PotT::bytes, pot_args(), pg, hc, loop);
   }
 
   // ---------------------------------------------------------- tensor maps
@@ -922,7 +914,7 @@ class Engine : public EngineBase {
   }
   // One iteration of the reference's `while itr < itrmax` loop.
   int couple_group(int set) {
-    if (use_pot()) return pot_group();
+    if (use_pot()) return pot_group(PotLoop{});
     const int n0 = g.n[0], h = g.h;
     (void)n0;
     const Box full = cube(g, 1 - h, h);
@@ -1086,8 +1078,13 @@ class Engine : public EngineBase {
     LCS_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     LCS_CUDA(cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     stream = side;
-    int rc2 = couple_group(set);
-    if (rc2 == LCS_OK)
+    int rc2 = LCS_OK;
+    if (use_pot()) {
+      for (int q = 0; q < pot_unroll() && rc2 == LCS_OK; q++) rc2 = pot_group(PotLoop{1, max_loop_groups(), handle});
+    } else {
+      rc2 = couple_group(set);
+    }
+    if (rc2 == LCS_OK && !use_pot())
       rc2 = launch("couple_continue", k_couple_continue, dim3(1), dim3(1), 0, dctx, handle, max_loop_groups());
     stream = main;
     cudaGraph_t body_out;
@@ -2134,7 +2131,7 @@ struct EngineGroup : GroupBase {
     if (rc2 == LCS_OK) {
       L->stream = side;
       L->grp = &mem;
-      rc2 = L->couple_group(set);
+      for (int q = 0; q < (L->use_pot() ? L->pot_unroll() : 1) && rc2 == LCS_OK; q++) rc2 = L->couple_group(set);
       if (rc2 == LCS_OK)
         rc2 = L->launch("couple_continue", k_group_continue<T>, dim3(1), dim3(1), 0, L->grp_ptrs, (int)mem.size(),
                         handle, L->max_loop_groups());

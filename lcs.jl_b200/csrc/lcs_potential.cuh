@@ -59,7 +59,7 @@ __device__ __forceinline__ float pot_div<float>(float x, float sx, float sy, flo
 
 constexpr int kPotLayers = 7;  // layers next to a face kept compact: n-2, n-1, n, 1, 2, 3, 4
 constexpr int kPotDLayers = 5; // of D along x: n-1, n, 1, 2, 3
-constexpr int kPotSlab = 26;   // output columns of a slab tile (32 less 3 on each side)
+constexpr int kPotSlab = 22;   // a slab tile's own columns (32 less 5 on each side)
 constexpr int kPotSlabThreads = 1024;
 
 // Layout of Phi and D (each in one of the spare velocity buffers): positions
@@ -117,6 +117,7 @@ struct PotGeom {
   int gx, gy;              // tile columns of k_pot_sweep along x and y
   int nseg, nc;            // CTAs; z chunks of a column
   int slab_part, nslab;    // residual partials of the slab tiles: first, count
+  int slab0[3];            // first tile of an axis's slabs (z, y, x in turn)
   double cx, cy, cz, k0, wd;  // 1/dx^2 .., 2 (cx + cy + cz), -omega dl
   double dxi, dyi, dzi;
 };
@@ -227,7 +228,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGroup<T> ga, PotGeom pg) {
   const int m = blockIdx.y;
   Ctx* ctx = ga.ctx[m];
-  if (ctx->cs.done || !ctx->pot_pending) return;
+  if (ctx->cs.done || !ctx->cs.cont || !ctx->pot_pending) return;
   const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz;
   T* D = pot_rhs<T>(ctx);
   T* s = ga.scratch[m];
@@ -286,33 +287,32 @@ __global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGro
   }
 }
 
-// The first sweep of an overlap group next to the faces normal to axis AX,
-// into the halo and the outer layers of Phi: the slabs (positions -1 .. 1 and
-// n+1 .. n+3), and of the core, which comes before them, the layers 2 and n
-// (both colours) and colour 0 of the layers 3 and n-1.  With these in place
-// k_pot_sweep leaves them alone in its first sweep and never needs the values
-// from before it: colour 0 of layer 4 reads colour 1 of layer 3, which is not
-// touched here, and colour 1 of layer 3 reads colour 0, which is final.
+// The first sweep of an overlap group next to the faces, into the halo and the
+// outer layers of Phi: the slabs (positions -1 .. 1 and n+1 .. n+3 along an
+// axis; z slabs first, then y, then x), and of the core, which comes before
+// them, the layers 2 and n (both colours) and colour 0 of the layers 3 and
+// n-1.  With these in place k_pot_sweep leaves them alone in its first sweep
+// and never needs the values from before it: colour 0 of layer 4 reads colour
+// 1 of layer 3, which is not touched here, and colour 1 of layer 3 reads
+// colour 0, which is final.
 //
-// A thread owns one column along AX through both slabs: the low one needs Phi
-// at -2 .. 4 and the high one at n-2 .. n+4, the same 7 images (n-2, n-1, n,
-// 1, 2, 3, 4; kept compact by k_pot_sweep, since along x they would be two
-// sectors of every row), and D at 5 of them.  Phases: colour 0 of the core
-// layers (2, 3 and n-1, n), colour 1 of the nearest, then the slab's two
-// colours; in-plane neighbours through shared memory, 3 barriers.  A tile of
-// 32 x 32 columns gives 26 x 26 (each half sweep needs one column more around).
-// Columns outside the slab's range are cells of the slabs done before (z
-// before y before x), as those left them.
+// A block takes 32 x 32 columns along one axis AX through both slabs: the low
+// one needs Phi at -2 .. 4 and the high one at n-2 .. n+4, the same 7 images
+// (n-2, n-1, n, 1, 2, 3, 4; kept compact by k_pot_sweep, since along x they
+// would be two sectors of every row), and D at 5 of them.  Phases, in-plane
+// neighbours through shared memory and a barrier between them: colours 0 and 1
+// of the core, then of the z slabs, the y slabs and the x slabs, as far as the
+// block's columns and its axis need them.  Blocks at the rim of a y or x slab
+// so sweep the few cells of the earlier slabs beside it themselves, and no
+// block waits for another: one launch instead of three (at 96^3 in FP32 the
+// three took 3 x 8 us).  A value reaches at most 5 columns (both colours of the
+// x, the y and the z slab, where the y slab crosses to the z slab in place),
+// so 22 x 22 of the columns are the block's own.
 template <typename T, int AX>
-__global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_constant__ PotGroup<T> ga, PotGeom pg,
-                                                              int part0) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[32];
-  const int m = blockIdx.z;
-  Ctx* ctx = ga.ctx[m];
-  if (ctx->cs.done || ctx->pot_redo) return;  // a group that runs again finds these in place
-  T* sh = (T*)smem_raw;  // [10][32][32]
+__device__ __forceinline__ void pot_slab_body(const PotGroup<T>& ga, const PotGeom& pg, int m, int tile, T* sh,
+                                              double* red) {
   constexpr int PL = 1024;
+  Ctx* ctx = ga.ctx[m];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = threadIdx.x;
   const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz;
   const int n[3] = {nx, ny, nz};
@@ -320,15 +320,21 @@ __global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_const
   const int nu = n[UA], nv = n[VA], nn = n[AX];
   const int ulo = AX == 0 ? 2 : -1, uhi = AX == 0 ? nu : nu + 3;
   const int vlo = AX == 2 ? -1 : 2, vhi = AX == 2 ? nv + 3 : nv;
-  const int u0 = ulo + blockIdx.x * kPotSlab, v0 = vlo + blockIdx.y * kPotSlab;
-  const int u = u0 - 3 + tx, v = v0 - 3 + ty;
+  const int gu = (uhi - ulo + kPotSlab) / kPotSlab;
+  const int u0 = ulo + (tile % gu) * kPotSlab - 5, v0 = vlo + (tile / gu) * kPotSlab - 5;
+  const int u = u0 + tx, v = v0 + ty;
   T* phi = pot_buf<T>(ctx, ctx->pot_cur);
   const T* D = pot_rhs<T>(ctx);
   const T* s = ga.scratch[m];
-  const int64_t face = (int64_t)nu * nv, f = (int64_t)(pot_wrap(v, nv) - 1) * nu + (pot_wrap(u, nu) - 1);
-  const bool inS = u >= ulo && u <= uhi && v >= vlo && v <= vhi;
-  const bool inC = u >= 2 && u <= nu && v >= 2 && v <= nv;
   const int uw = pot_wrap(u, nu), vw = pot_wrap(v, nv);
+  const int64_t face = (int64_t)nu * nv, f = (int64_t)(vw - 1) * nu + (uw - 1);
+  const bool mine = tx >= 5 && tx < 5 + kPotSlab && ty >= 5 && ty < 5 + kPotSlab && u <= uhi && v <= vhi;
+  // what the column's cells are: its place in the core and in the slabs of the two other axes
+  const bool uc = u >= 2 && u <= nu, vc = v >= 2 && v <= nv;
+  const bool ur = u >= -1 && u <= nu + 3, vr = v >= -1 && v <= nv + 3;
+  const bool isC = uc && vc;
+  const bool isZ = AX == 2 ? ur && vr : ur && vr && !vc;
+  const bool isY = AX == 1 ? ur && vc : AX == 0 && ur && !uc && vc;
   T lo[7], hi[7], d[5];
   // images n-2, n-1, n, 1, 2, 3, 4 of the column
 #pragma unroll
@@ -347,111 +353,79 @@ __global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_const
       }
     }
   }
-  if constexpr (AX != 2) {
-    // columns of the slabs swept before: their cells inside this slab's layers
-    const bool zc = v == 1 || v == nv + 1;
-    const bool yc = AX == 0 && !zc && (u == 1 || u == nu + 1);
-    const bool ok = AX == 1 ? (zc && u >= -1 && u <= nx + 3)
-                            : ((zc && u >= -1 && u <= ny + 3) || (yc && v >= 2 && v <= nz));
-    if (ok) {
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        const int pl = q - 1, ph = nn + 1 + q;  // positions along AX
-        lo[1 + q] = phi[AX == 1 ? pg.s.at(u, pl, v) : pg.s.at(pl, u, v)];
-        hi[3 + q] = phi[AX == 1 ? pg.s.at(u, ph, v) : pg.s.at(ph, u, v)];
-      }
-    }
-  }
   const T cu = (T)(UA == 0 ? pg.cx : pg.cy), cv = (T)(VA == 1 ? pg.cy : pg.cz),
           cn = (T)(AX == 0 ? pg.cx : AX == 1 ? pg.cy : pg.cz), k0 = (T)pg.k0, wd = (T)pg.wd;
-  // planes in shared memory: core layers lo 4, lo 5, hi 1, hi 2, then the slab layers lo 1-3, hi 3-5
-  sh[0 * PL + c] = lo[4];
-  sh[1 * PL + c] = lo[5];
-  sh[2 * PL + c] = hi[1];
-  sh[3 * PL + c] = hi[2];
+  // planes in shared memory: lo 1 .. 5, then hi 1 .. 5
 #pragma unroll
-  for (int q = 0; q < 3; q++) {
-    sh[(4 + q) * PL + c] = lo[1 + q];
-    sh[(7 + q) * PL + c] = hi[3 + q];
+  for (int q = 0; q < 5; q++) {
+    sh[q * PL + c] = lo[1 + q];
+    sh[(5 + q) * PL + c] = hi[1 + q];
   }
-  __syncthreads();
   const int cl = tx > 0 ? c - 1 : c, cr = tx < 31 ? c + 1 : c, cd = ty > 0 ? c - 32 : c, cup = ty < 31 ? c + 32 : c;
   const int par = (u + v) & 1;
-  // one cell: layer q of `a` at position parity pp; its plane in shared memory
-  auto relax = [&](T* a, int q, int plane) -> T {
-    const T* p = sh + plane * PL;
+  double acc = 0.0;
+  // one cell: layer q of `a`, in shared memory in the planes from `base`
+  // (cells of one colour never read each other: in place)
+  auto relax = [&](T* a, int q, int base, bool count) {
+    T* p = sh + (base + q - 1) * PL;
     const T su = p[cl] + p[cr], sv = p[cd] + p[cup], sn = a[q - 1] + a[q + 1];
     const T div = pot_div<T>(a[q], su, sv, sn, d[q - 1], cu, cv, cn, k0);
     a[q] = pfma<T>(wd, div, a[q]);
-    return div;
+    p[c] = a[q];
+    if (count) acc += (double)div * (double)div;
   };
   // positions: lo q -> q - 2, hi q -> n - 2 + q (n even): both have the parity of q
-  auto color = [&](int q) { return (par + q) & 1; };
-  const bool mine = tx >= 3 && tx < 3 + kPotSlab && ty >= 3 && ty < 3 + kPotSlab;
-  // core cells of these layers that an earlier slab's launch counts in the residual
+  auto has = [&](int q, int color) { return ((par + q) & 1) == color; };
+  // core cells of these layers that belong to an axis before this one: it
+  // stores them and counts them in the residual (each cell once, whatever the
+  // order of the blocks)
   auto outer = [&](int p, int pn, int c0) { return p == 2 || p == pn || (c0 == 0 && (p == 3 || p == pn - 1)); };
-  auto counts = [&](int c0) {
-    return mine && !(AX != 2 && outer(v, nv, c0)) && !(AX == 0 && outer(u, nu, c0));
+  auto own_core = [&](int c0) { return mine && isC && !(AX != 2 && outer(v, nv, c0)) && !(AX == 0 && outer(u, nu, c0)); };
+  // a colour of the slab cells: lo 1-3, hi 3-5 (this axis's own slabs), or of
+  // the columns in another slab: all layers
+  auto slab = [&](bool is, int color, bool own) {
+    __syncthreads();
+    if (!is) return;
+    const bool count = own && mine && u >= 1 && u <= nu + 1 && v >= 1 && v <= nv + 1;  // cells 1 and n+1 count
+#pragma unroll
+    for (int q = 1; q <= 5; q++)
+      if (has(q, color) && (q <= 3 || !own)) relax(lo, q, 0, count && q == 3);
+#pragma unroll
+    for (int q = 1; q <= 5; q++)
+      if (has(q, color) && (q >= 3 || !own)) relax(hi, q, 5, count && q == 3);
   };
-  double acc = 0.0;
-  auto add = [&](T r) { acc += (double)r * (double)r; };
-  if (inC) {  // colour 0 of the core layers
-    const bool cnt = counts(0);
-    T r0, r1;
-    if (color(4) == 0) {
-      r0 = relax(lo, 4, 0);
-      r1 = relax(hi, 2, 3);
+  __syncthreads();
+  if (isC) {  // colour 0 of the core layers 2, 3 and n-1, n
+    const bool count = own_core(0);
+    if (has(4, 0)) {
+      relax(lo, 4, 0, count);
+      relax(hi, 2, 5, count);
     } else {
-      r0 = relax(lo, 5, 1);
-      r1 = relax(hi, 1, 2);
+      relax(lo, 5, 0, count);
+      relax(hi, 1, 5, count);
     }
-    if (cnt) {
-      add(r0);
-      add(r1);
-    }
-  }
-  if (color(4) == 0) {  // for colour 1 next to it (cells of one colour never read each other)
-    sh[0 * PL + c] = lo[4];
-    sh[3 * PL + c] = hi[2];
   }
   __syncthreads();
-  if (inC && color(4) == 1) {
-    const T r0 = relax(lo, 4, 0), r1 = relax(hi, 2, 3);
-    if (counts(1)) {
-      add(r0);
-      add(r1);
+  if (isC && has(4, 1)) {  // colour 1 of the layers 2 and n
+    const bool count = own_core(1);
+    relax(lo, 4, 0, count);
+    relax(hi, 2, 5, count);
+  }
+  if (AX == 2 || v0 <= 1 || v0 + 31 > nv) {  // (the same for the whole block)
+    slab(isZ, 0, AX == 2);
+    slab(isZ, 1, AX == 2);
+  }
+  if constexpr (AX != 2) {
+    if (AX == 1 || u0 <= 1 || u0 + 31 > nu) {
+      slab(isY, 0, AX == 1);
+      slab(isY, 1, AX == 1);
     }
   }
-  // slab cells: lo 1-3 (positions -1 .. 1), hi 3-5 (n+1 .. n+3)
-  const bool ownr = inS && mine && u >= 1 && u <= nu + 1 && v >= 1 && v <= nv + 1;  // cells 1 and n+1 count in the residual
-#pragma unroll
-  for (int color_of = 0; color_of < 2; color_of++) {
-    if (inS) {
-#pragma unroll
-      for (int q = 1; q <= 3; q++)
-        if (color(q) == color_of) {
-          const T r = relax(lo, q, 3 + q);
-          if (q == 3 && ownr) add(r);
-        }
-#pragma unroll
-      for (int q = 3; q <= 5; q++)
-        if (color(q) == color_of) {
-          const T r = relax(hi, q, 4 + q);
-          if (q == 3 && ownr) add(r);
-        }
-    }
-    if (color_of == 0) {
-      if (inS) {
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-          if (color(1 + q) == 0) sh[(4 + q) * PL + c] = lo[1 + q];
-          if (color(3 + q) == 0) sh[(7 + q) * PL + c] = hi[3 + q];
-        }
-      }
-      __syncthreads();
-    }
+  if constexpr (AX == 0) {
+    slab(isC, 0, true);
+    slab(isC, 1, true);
   }
-  if (inS && mine) {
+  if (mine) {
     auto put = [&](int p, T val) {
       phi[AX == 2 ? pg.s.at(u, v, p) : AX == 1 ? pg.s.at(u, p, v) : pg.s.at(p, u, v)] = val;
     };
@@ -460,17 +434,31 @@ __global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_const
       put(q - 1, lo[1 + q]);
       put(nn + 1 + q, hi[3 + q]);
     }
-    if (inC) {
+    if (own_core(has(4, 0) ? 0 : 1)) {
       put(2, lo[4]);
       put(nn, hi[2]);
-      if (color(5) == 0) {
-        put(3, lo[5]);
-        put(nn - 1, hi[1]);
-      }
+    }
+    if (has(5, 0) && own_core(0)) {
+      put(3, lo[5]);
+      put(nn - 1, hi[1]);
     }
   }
   const double sum = block_sum<kPotSlabThreads>(acc, red);
-  if (threadIdx.x == 0) ga.partials[m][part0 + blockIdx.y * gridDim.x + blockIdx.x] = sum;
+  if (threadIdx.x == 0) ga.partials[m][pg.slab_part + blockIdx.x] = sum;
+}
+// blocks: the tiles of the z slabs, then of the y and x slabs (slab0: first tile of each axis)
+template <typename T>
+__global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_constant__ PotGroup<T> ga, PotGeom pg) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[32];
+  const int m = blockIdx.y, b = blockIdx.x;
+  const Ctx* ctx = ga.ctx[m];
+  // (a group that runs again finds these in place)
+  if (ctx->cs.done || !ctx->cs.cont || ctx->pot_redo) return;
+  T* sh = (T*)smem_raw;  // [10][32][32]
+  if (b < pg.slab0[1]) pot_slab_body<T, 2>(ga, pg, m, b, sh, red);
+  else if (b < pg.slab0[0]) pot_slab_body<T, 1>(ga, pg, m, b - pg.slab0[1], sh, red);
+  else pot_slab_body<T, 0>(ga, pg, m, b - pg.slab0[0], sh, red);
 }
 
 constexpr int kPotMaxChunk = 1024, kPotMaxPlanes = kPotMaxChunk + 24;
@@ -490,6 +478,14 @@ struct PotTile {
   static constexpr size_t x_elems = (size_t)2 * 6 * NW * 2 * 32; // rows at the warps' edges, double buffered
   static constexpr size_t bytes = (d_elems + x_elems) * sizeof(T) + kPotMaxPlanes * sizeof(int);
   static_assert(RW % 2 == 0, "a warp's first row has the same parity in every warp");
+};
+
+// The loop of a couple inside a step graph: the last CTA of a group's sweep
+// sets its condition (a run alone; a batch group has a kernel for it, which
+// looks at all its members).
+struct PotLoop {
+  int on, max_groups;
+  cudaGraphConditionalHandle handle;
 };
 
 // Three red-black sweeps (six half sweeps) in one pass.
@@ -514,7 +510,7 @@ struct PotTile {
 // (pairs never straddle the period: n is even).
 template <typename T, int NW, int RW>
 __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
-    k_pot_sweep(const __grid_constant__ PotGroup<T> ga, PotGeom pg, HsmacCoef cf, int group_end) {
+    k_pot_sweep(const __grid_constant__ PotGroup<T> ga, PotGeom pg, HsmacCoef cf, PotLoop loop) {
   using L = PotTile<T, NW, RW>;
   using T2 = pair_t<T>;
   constexpr int UF = 2;  // planes between two moves of the registers
@@ -527,7 +523,7 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   int* sZ = (int*)((T*)smem_raw + L::d_elems + L::x_elems);  // box bits of the planes kb - 13 ..
   const int m = blockIdx.y;
   Ctx* ctx = ga.ctx[m];
-  if (ctx->cs.done) return;
+  if (ctx->cs.done || !ctx->cs.cont) return;
   const int cur = ctx->pot_cur, redo = ctx->pot_redo;
   const int nsw = redo ? redo : 3;  // sweeps of this pass
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -652,12 +648,6 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
       dbase[s6 + DS + r * 32] = Lft ? dr : dl;
     }
     load_plane(min(t + 1, kend));
-#ifdef PSPLIT
-    if (t > ks) {
-      if (!mbar_wait_bounded(&ebar, epar)) ctx->wait_error = 1;
-      epar ^= 1;
-    }
-#endif
     auto half = [&](auto h_tag) {
       constexpr int H = decltype(h_tag)::value;
       constexpr int I = I0 + H, SW = (H - 1) / 2, BIT = H <= 2 ? H - 1 : SW + 1;
@@ -701,10 +691,6 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
       xout[h * NW * 64] = Y[0][I0 + h];
       xout[h * NW * 64 + 32] = Y[RW - 1][I0 + h];
     }
-#ifdef PSPLIT
-    __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ebar)) : "memory");
-#endif
     // plane t - 6
     const int q = t - 6;
     if (FULL || (q >= kb && q <= ke)) {
@@ -747,9 +733,7 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
 #pragma unroll
     for (int h = 5; h > 0; h--) slot[h] = slot[h - 1];
     slot[0] = s6;
-#ifndef PSPLIT
     __syncthreads();
-#endif
   };
 
   using T_ = std::true_type;
@@ -773,10 +757,6 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
       }
   }
 
-#ifdef PSPLIT
-  mbar_wait_bounded(&ebar, epar);
-  epar ^= 1;
-#endif
   // residuals of the pass's sweeps; the last CTA runs the exit tests
   const unsigned int nb = gridDim.x;
   double* part = ga.partials[m];
@@ -800,7 +780,7 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   int again = 0;  // the exit lies inside the group: run it again up to that sweep
   if (redo == 0) {
     for (int q = 0; q < 3; q++) {
-      hsmac_check(ctx, cf, sum[q] + ctx->pot_floor * cf.count, group_end);
+      hsmac_check(ctx, cf, sum[q] + ctx->pot_floor * cf.count, 1);
       if (ctx->cs.done) {
         if (q < 2 && isfinite(ctx->cs.div)) again = q + 1;
         break;
@@ -817,6 +797,7 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   ctx->pot_redo = again;
   ctx->pot_pending = again ? 0 : 1;
   if (!again) ctx->pot_cur = 1 - cur;
+  if (loop.on) cudaGraphSetConditional(loop.handle, couple_goes_on(ctx, loop.max_groups) ? 1u : 0u);
 }
 
 // End of a couple: the velocity and P from Phi.  Bound by HBM: 5 fields read,
