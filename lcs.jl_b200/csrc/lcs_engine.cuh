@@ -328,13 +328,17 @@ class Engine : public EngineBase {
   bool pot_ok = false;
   int debug_kind = 0;
   bool use_pot() const { return pot_ok && debug_kind == 0; }
-    // tile of the sweep: FP64 8 warps of 4 rows.  FP32 12 warps of 4 rows on
-  // grids of more than 256^3 cells, where fewer redundant rows count, and 16 of
-  // 2 rows up to there, where a plane's latency does.
-  static constexpr int kPotR = 4, kPotW = sizeof(T) == 8 ? 8 : 12, kPotRS = sizeof(T) == 8 ? 4 : 2, kPotWS = sizeof(T) == 8 ? 8 : 16;
-  bool pot_small = true;
-  using PotT = PotTile<T, kPotW, kPotR>;
-  using PotS = PotTile<T, kPotWS, kPotRS>;
+    // Tiles of the sweep (warps x rows a warp).  Taller tiles do less redundant
+  // work, a plane of shorter ones takes less time, and a grid of few tiles
+  // leaves SMs idle that shorter ones would use; pot_geom weighs them by the
+  // time of a plane.  Measured, us a launch with tiles of 36, 20 and 4 rows
+  // (FP64: 20 and 4): FP32 32^3 33, 27, 21; 48^3 33, 27, 24; 64^3 35, 31, 35;
+  // 96^3 43, 37, 64; 128^3 60, 56, 122; 192^3 117, 127, 273; 256^3 240, 228;
+  // 512^3 1044, 1199.  FP64 48^3 33, 29; 64^3 40, 41; 96^3 52, 77.
+  static constexpr int kPotW = sizeof(T) == 8 ? 8 : 12, kPotWS = sizeof(T) == 8 ? 8 : 16, kPotRS = sizeof(T) == 8 ? 4 : 2;
+  using PotT = PotTile<T, kPotW, 4>;        // FP64 20 output rows, FP32 36
+  using PotS = PotTile<T, kPotWS, kPotRS>;  // FP32 20 output rows (FP64: the same as PotT)
+  using PotV = PotTile<T, 8, 2>;            // 4 output rows
   static constexpr size_t kSlabSmem = (size_t)10 * 1024 * sizeof(T);
   int init_pot() {
     const char* sweep = std::getenv("LCS_B200_FUSED_SWEEP");
@@ -348,11 +352,9 @@ class Engine : public EngineBase {
              (size_t)ps.total * sizeof(T) <= (size_t)plan.stage_elems * sizeof(double) &&
              (sw == "potential" || (sw.empty() && !shaped && (sizeof(T) == 4 || cells > 40 * 40 * 40)));
     if (!pot_ok) return LCS_OK;
-    pot_small = cells <= 256 * 256 * 256;
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotW, kPotR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)PotT::bytes));
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotWS, kPotRS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)PotS::bytes));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotW, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotT::bytes));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotWS, kPotRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotS::bytes));
+    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotV::bytes));
     LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
     pot_ptrs.ctx[0] = dctx;
     pot_ptrs.P[0] = P;
@@ -365,22 +367,30 @@ class Engine : public EngineBase {
     memset(&pg, 0, sizeof pg);
     pg.s = pot_scratch(g.n, (int)sizeof(T));
     pg.overlap = cfg.overlap ? 1 : 0;
-    const int ty = pot_small ? PotS::TY : PotT::TY;
-    pg.gx = (g.n[0] + 1 + PotT::TX - 1) / PotT::TX;
-    pg.gy = (g.n[1] + 1 + ty - 1) / ty;
     // A CTA takes one of nc z chunks of a tile column; its time is its planes
-    // and the 12 more that fill and drain the six half sweeps.
-    const int cols = pg.gx * pg.gy, nu = (g.n[2] + 2) / 2, slots = share_slots(num_sms);
-    double best = 1e300;
+    // and the 12 more that fill and drain the six half sweeps, times the
+    // measured time of a plane.
+    const int nu = (g.n[2] + 2) / 2, slots = share_slots(num_sms);
     const int cu = zchunk_force > 0 ? (zchunk_force + 1) / 2 : 0;  // units of two planes of a forced chunk
-    for (int nc = std::max(cu > 0 ? (nu + cu - 1) / cu : 1, (2 * nu + kPotMaxChunk - 1) / kPotMaxChunk); nc <= nu; nc++) {
-      const double cost = std::ceil((double)cols * nc / slots) * (2.0 * ((nu + nc - 1) / nc) + 12.0);
-      if (cost < best - 1e-9) {
-        best = cost;
-        pg.nc = nc;
-        pg.nseg = cols * nc;
+    pg.gx = (g.n[0] + 1 + PotT::TX - 1) / PotT::TX;
+    const int rows[3] = {PotT::TY, PotS::TY, PotV::TY};
+    const double plane_us[3] = {sizeof(T) == 8 ? 2.1 : 2.2, sizeof(T) == 8 ? 2.1 : 1.5, sizeof(T) == 8 ? 1.15 : 0.92};
+    double best = 1e300;
+    const char* force = std::getenv("LCS_B200_POT_TILE");  // 0, 1 or 2 (the tests and timing): that tile
+    for (int kind = 0; kind < 3; kind++) {
+      if (force && std::atoi(force) != kind) continue;
+      const int gy = (g.n[1] + 1 + rows[kind] - 1) / rows[kind], cols = pg.gx * gy;
+      for (int nc = std::max(cu > 0 ? (nu + cu - 1) / cu : 1, (2 * nu + kPotMaxChunk - 1) / kPotMaxChunk); nc <= nu; nc++) {
+        const double cost = std::ceil((double)cols * nc / slots) * (2.0 * ((nu + nc - 1) / nc) + 12.0) * plane_us[kind];
+        if (cost < best - 1e-9) {
+          best = cost;
+          pg.kind = kind;
+          pg.gy = gy;
+          pg.nc = nc;
+          pg.nseg = cols * nc;
+        }
+        if (cu > 0 || (int64_t)cols * nc > 64 * (int64_t)slots) break;
       }
-      if (cu > 0 || (int64_t)cols * nc > 64 * (int64_t)slots) break;
     }
     pg.slab_part = 3 * pg.nseg;
     if (cfg.overlap)
@@ -423,9 +433,12 @@ class Engine : public EngineBase {
     LCS_TRY(launch("pot_jump", k_pot_jump<T>, dim3(blocks_for(faces, 256), M), dim3(256), 0, pot_args(), pg));
     if (cfg.overlap)
       LCS_TRY(launch("pot_slab", k_pot_slab<T>, dim3(pg.nslab, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg));
-    if (pot_small)
-      return launch("pot_sweep", k_pot_sweep<T, kPotWS, kPotRS>, dim3(pg.nseg, M), dim3(PotS::NT), PotS::bytes, pot_args(), pg, hc, loop);
-    return launch("pot_sweep", k_pot_sweep<T, kPotW, kPotR>, dim3(pg.nseg, M), dim3(PotT::NT), PotT::bytes, pot_args(), pg, hc, loop);
+    const dim3 grid(pg.nseg, M);
+    if (pg.kind == 2)
+      return launch("pot_sweep", k_pot_sweep<T, 8, 2>, grid, dim3(PotV::NT), PotV::bytes, pot_args(), pg, hc, loop);
+    if (pg.kind == 1)
+      return launch("pot_sweep", k_pot_sweep<T, kPotWS, kPotRS>, grid, dim3(PotS::NT), PotS::bytes, pot_args(), pg, hc, loop);
+    return launch("pot_sweep", k_pot_sweep<T, kPotW, 4>, grid, dim3(PotT::NT), PotT::bytes, pot_args(), pg, hc, loop);
   }
 
   // ---------------------------------------------------------- tensor maps

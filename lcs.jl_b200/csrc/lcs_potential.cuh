@@ -114,7 +114,7 @@ struct PotGroup {
 struct PotGeom {
   PotScratch s;
   int overlap;
-  int gx, gy;              // tile columns of k_pot_sweep along x and y
+  int kind, gx, gy;        // tile of k_pot_sweep (host's choice), tile columns along x and y
   int nseg, nc;            // CTAs; z chunks of a column
   int slab_part, nslab;    // residual partials of the slab tiles: first, count
   int slab0[3];            // first tile of an axis's slabs (z, y, x in turn)

@@ -58,6 +58,20 @@ def test_fp64_equals_the_element_wise_order(dims, ov):
         assert rel_l2(a, b) <= 1e-12
 
 
+@pytest.mark.parametrize("tile", ["0", "1", "2"])
+@pytest.mark.parametrize("dims", [(24, 26, 30), (54, 38, 66), (106, 74, 16)])
+def test_sweep_tiles(dims, tile, monkeypatch):
+    """The three tile heights (FP64: two) on the same grids."""
+    monkeypatch.setenv("LCS_B200_POT_TILE", tile)
+    _, g = couple(Engine, dims, True, 6, 12, 1e-12)
+    _, o = couple(OracleEngine, dims, True, 6, 12, 1e-12)
+    for a, b in zip(g, o):
+        assert rel_l2(a, b) <= 1e-12
+    _, f = couple(Engine, dims, True, 6, 12, 1e-12, F.PRECISION_FP32_MIXED)
+    errs = [rel_l2(a, b) for a, b in zip(f, o)]
+    assert max(errs[:3]) <= 1e-5 and errs[3] <= 1e-3, errs
+
+
 @pytest.mark.parametrize("itrmin", [6, 7, 8])
 @pytest.mark.parametrize("itrmax", [9, 60])
 @pytest.mark.parametrize("ov", [True, False])
@@ -73,7 +87,6 @@ def test_exit_inside_a_group(itrmin, itrmax, ov):
 
 @pytest.mark.parametrize("dims", [(24, 26, 30), (54, 38, 20), (272, 250, 252)])
 def test_fp32_close_to_fp64(dims):
-    """(272, 250, 252) has more than 256^3 cells: the taller FP32 tiles."""
     l32, a = couple(Engine, dims, True, 6, 12, 1e-12, F.PRECISION_FP32_MIXED)
     l64, b = couple(Engine, dims, True, 6, 12, 1e-12)
     assert l32["sweeps"] == l64["sweeps"]
