@@ -1878,10 +1878,14 @@ class Engine : public EngineBase {
     LCS_TRY(copy(d_edges, out->edges, (size_t)(nbins + 1) * 8, cudaMemcpyHostToDevice));
     LCS_CUDA(cudaMemsetAsync(d_counts, 0, (size_t)(nbins + 1) * 8, stream));
     const size_t rdf_smem = (size_t)(nbins + 1) * 16;
+    // no pair further apart counts (a margin for the roundings of d and d / diam)
+    const double reach = std::fmax(out->edges[nbins], dm * (1.0 + pc->contact_tolerance)) * (1.0 + 1e-9);
+    const int prune = out->x.min >= 0.0 && out->y.min >= 0.0 && out->z.min >= 0.0 && out->x.max <= kDomainLength &&
+                      out->y.max <= kDomainLength && out->z.max <= kDomainLength;
     LCS_TRY(launch("rdf", k_rdf, dim3(blocks_for(n, 256, 148 * 8)), dim3(256), rdf_smem, (const double*)sp[s].p[0],
                    (const double*)sp[s].p[1], (const double*)sp[s].p[2], (const int64_t*)(sp[s].p[0] + 16 * n),
                    (const int64_t*)c.hashes, (const int64_t*)c.starts, (const int64_t*)(c.starts + c.H), n, c.cg,
-                   pc->search_cell_size, (const double*)d_edges, nbins, dm, pc->contact_tolerance, d_counts));
+                   pc->search_cell_size, (const double*)d_edges, nbins, dm, pc->contact_tolerance, reach, prune, d_counts));
     std::vector<unsigned long long> counts(nbins + 1);
     LCS_TRY(copy(counts.data(), d_counts, (size_t)(nbins + 1) * 8, cudaMemcpyDeviceToHost));
     // the spectrum (spectrum.jl:11-78)
@@ -1893,9 +1897,9 @@ class Engine : public EngineBase {
       double* d_part = d_k + (size_t)npairs * 3;
       double* d_sums = d_part + (size_t)nbx * npairs * 2;
       LCS_TRY(copy(d_k, kvec.data(), (size_t)npairs * 3 * 8, cudaMemcpyHostToDevice));
-      const unsigned int nby = (unsigned)((npairs + 256 * kSpecPairs - 1) / (256 * kSpecPairs));
+      const unsigned int nby = (unsigned)((ns + kSpecDirs - 1) / kSpecDirs);
       LCS_TRY(launch("spectrum", k_spectrum, dim3(nbx, nby), dim3(256), 0, (const double*)sp[s].p[0],
-                     (const double*)sp[s].p[1], (const double*)sp[s].p[2], n, (const double*)d_k, npairs, d_part));
+                     (const double*)sp[s].p[1], (const double*)sp[s].p[2], n, (const double*)d_k, nshells, ns, d_part));
       LCS_TRY(launch("spectrum_final", k_spectrum_final, dim3((unsigned)((2 * npairs + 255) / 256)), dim3(256), 0,
                      (const double*)d_part, (int)nbx, npairs, d_sums));
       LCS_TRY(copy(sums.data(), d_sums, (size_t)npairs * 2 * 8, cudaMemcpyDeviceToHost));

@@ -17,6 +17,7 @@
 // atomics, in no fixed order).
 #pragma once
 
+#include "../../include/lcs_b200.h"
 #include "lcs_common.cuh"
 #include "lcs_makeindex.cuh"
 
@@ -84,12 +85,22 @@ __device__ __forceinline__ double dist3(double x1, double y1, double z1, double 
 // Pairs (id1 < id2) per bin k (edges[k] < d <= edges[k+1], the bin of
 // searchsortedfirst(edges, d) - 1) and contact pairs |d / diam - 1| < tol.
 // Dynamic shared memory: nbins + 1 counters, then nbins + 1 edges.
+//
+// No pair further apart than `reach` (a little over the last edge and the
+// contact distance) counts, and nearly all candidates are: with the production
+// settings the last edge is half a cell, so of the 125 cells within 2 of a
+// particle's own a sphere of 0.4 % counts.  The square is compared before the
+// root, the bin search and the division, and `prune` (every particle lies in
+// the box, so every particle of a cell does lie in it) skips the cells that
+// are further away; the cells of a row along x are one run of particles.
+// 2^20 particles at 256^3 with the production settings: the statistics call
+// took 10.5 ms and takes 2.1 (with the spectrum below).
 __global__ void __launch_bounds__(256) k_rdf(const double* __restrict__ X, const double* __restrict__ Y,
                                              const double* __restrict__ Z, const int64_t* __restrict__ ids,
                                              const int64_t* __restrict__ hashes, const int64_t* __restrict__ starts,
                                              const int64_t* __restrict__ stops, int64_t n, CellGeom cg, int ncell,
                                              const double* __restrict__ edges_g, int nbins, double diam, double tol,
-                                             unsigned long long* __restrict__ counts) {
+                                             double reach, int prune, unsigned long long* __restrict__ counts) {
   extern __shared__ unsigned long long rdf_sh[];
   unsigned long long* hist = rdf_sh;                   // [0, nbins): bins, [nbins]: contact
   double* edges = (double*)(rdf_sh + nbins + 1);       // nbins + 1
@@ -105,38 +116,45 @@ __global__ void __launch_bounds__(256) k_rdf(const double* __restrict__ X, const
     if (c1[0] < 1 || c1[0] > cg.nc[0] || c1[1] < 1 || c1[1] > cg.nc[1] || c1[2] < 1 || c1[2] > cg.nc[2]) continue;
     const double x1 = X[i1], y1 = Y[i1], z1 = Z[i1];
     const int64_t id1 = ids[i1];
-    for (int di = -ncell; di <= ncell; di++) {
-      const int a = c1[0] + di;
-      if (a < 0 || a > cg.nc[0] + 1) continue;
-      for (int dj = -ncell; dj <= ncell; dj++) {
-        const int b = c1[1] + dj;
-        if (b < 0 || b > cg.nc[1] + 1) continue;
-        for (int dk = -ncell; dk <= ncell; dk++) {
-          const int c = c1[2] + dk;
-          if (c < 0 || c > cg.nc[2] + 1) continue;
-          const int64_t h2 = 1 + a + b * W + c * WH;
-          const int64_t lo = starts[h2 - 1], hi = stops[h2 - 1];  // 1-based, inclusive
-          for (int64_t i2 = lo; i2 <= hi; i2++) {
-            if (!(id1 < ids[i2 - 1])) continue;
-            const double d = dist3(x1, y1, z1, X[i2 - 1], Y[i2 - 1], Z[i2 - 1]);
-            // searchsortedfirst(edges, d): first 1-based index with edges >= d
-            int lo_e = 0, len = nbins + 1;
-            while (len > 0) {
-              const int half = len >> 1;
-              if (edges[lo_e + half] < d) {
-                lo_e += half + 1;
-                len -= half + 1;
-              } else {
-                len = half;
-              }
-            }
-            const int k = lo_e;  // = searchsortedfirst - 1 (1-based bin), 0-based: k - 1
-            if (k >= 1 && k <= nbins) atomicAdd(&hist[k - 1], 1ull);
-            if (fabs(__dsub_rn(d / diam, 1.0)) < tol) atomicAdd(&hist[nbins], 1ull);
-          }
-        }
+    // the neighbour cells along an axis: within ncell, inside the axes, and
+    // (prune) with a near side closer than reach
+    const double p1[3] = {x1, y1, z1};
+    int lo3[3], hi3[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      lo3[a] = max(c1[a] - ncell, 0);
+      hi3[a] = min(c1[a] + ncell, cg.nc[a] + 1);
+      if (prune) {
+        const double far = reach + 1e-9;
+        while (lo3[a] < c1[a] && p1[a] - lo3[a] * cg.dxc[a] > far) lo3[a]++;
+        while (hi3[a] > c1[a] && (hi3[a] - 1) * cg.dxc[a] - p1[a] > far) hi3[a]--;
       }
     }
+    for (int c = lo3[2]; c <= hi3[2]; c++)
+      for (int b = lo3[1]; b <= hi3[1]; b++) {
+        const int64_t row = b * W + c * WH;  // hash - 1 of the row's cell 0
+        const int64_t lo = starts[row + lo3[0]], hi = stops[row + hi3[0]];  // 1-based, inclusive
+        for (int64_t i2 = lo; i2 <= hi; i2++) {
+          const double ex = __dsub_rn(x1, X[i2 - 1]), ey = __dsub_rn(y1, Y[i2 - 1]), ez = __dsub_rn(z1, Z[i2 - 1]);
+          const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
+          if (d2 > reach * reach || !(id1 < ids[i2 - 1])) continue;
+          const double d = sqrt(d2);  // dist3
+          // searchsortedfirst(edges, d): first 1-based index with edges >= d
+          int lo_e = 0, len = nbins + 1;
+          while (len > 0) {
+            const int half = len >> 1;
+            if (edges[lo_e + half] < d) {
+              lo_e += half + 1;
+              len -= half + 1;
+            } else {
+              len = half;
+            }
+          }
+          const int k = lo_e;  // = searchsortedfirst - 1 (1-based bin), 0-based: k - 1
+          if (k >= 1 && k <= nbins) atomicAdd(&hist[k - 1], 1ull);
+          if (fabs(__dsub_rn(d / diam, 1.0)) < tol) atomicAdd(&hist[nbins], 1ull);
+        }
+      }
   }
   __syncthreads();
   for (int k = threadIdx.x; k <= nbins; k += blockDim.x)
@@ -144,29 +162,31 @@ __global__ void __launch_bounds__(256) k_rdf(const double* __restrict__ X, const
 }
 
 // Spectrum sums: block (bx, by) adds cos and sin of k.x over its particle
-// chunk for the pairs [by * 256 * kSpecPairs, ...) (thread t: pairs t + 256 j),
-// particles staged in shared memory; partials[(bx * npairs + pair) * 2 + {0,1}].
-constexpr int kSpecPairs = 4;
+// chunk for the directions [by * 64, ...) and every shell; thread t takes
+// direction t mod 64 and every fourth particle of a tile staged in shared
+// memory; partials[(bx * npairs + shell * ns + direction) * 2 + {0,1}].
+//
+// The wavenumbers are 1, 2, 3 and then twice the one two before (4 = 2 x 2,
+// 6 = 2 x 3, 8 = 2 x 4, ...), all along the same directions, so the phase
+// factors of all shells are products of that of wavenumber 1: one sincos and a
+// squaring per shell instead of a sincos per shell.  The error of a phase
+// grows with the wavenumber either way (k.x is rounded at its own size).
+constexpr int kSpecDirs = 64;
 constexpr int kSpecTile = 512;
 __global__ void __launch_bounds__(256) k_spectrum(const double* __restrict__ X, const double* __restrict__ Y,
                                                   const double* __restrict__ Z, int64_t n,
-                                                  const double* __restrict__ kvec, int npairs,
+                                                  const double* __restrict__ kvec, int nshells, int ns,
                                                   double* __restrict__ partials) {
   __shared__ double px[kSpecTile], py[kSpecTile], pz[kSpecTile];
+  __shared__ double red[2][256];
   const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
   const int64_t p0 = (int64_t)blockIdx.x * chunk, p1 = p0 + chunk < n ? p0 + chunk : n;
-  double kx[kSpecPairs], ky[kSpecPairs], kz[kSpecPairs], ac[kSpecPairs], as[kSpecPairs];
-  int pr[kSpecPairs];
+  const int dir = blockIdx.y * kSpecDirs + threadIdx.x % kSpecDirs, sub = threadIdx.x / kSpecDirs;
+  const int q = dir < ns ? dir : 0;  // kvec's first ns entries: wavenumber 1
+  const double kx = kvec[3 * q], ky = kvec[3 * q + 1], kz = kvec[3 * q + 2];
+  double ac[LCS_SPECTRUM_MAX_SHELLS], as[LCS_SPECTRUM_MAX_SHELLS];
 #pragma unroll
-  for (int j = 0; j < kSpecPairs; j++) {
-    pr[j] = blockIdx.y * 256 * kSpecPairs + threadIdx.x + 256 * j;
-    const int q = pr[j] < npairs ? pr[j] : 0;
-    kx[j] = kvec[3 * q];
-    ky[j] = kvec[3 * q + 1];
-    kz[j] = kvec[3 * q + 2];
-    ac[j] = 0.0;
-    as[j] = 0.0;
-  }
+  for (int b = 0; b < LCS_SPECTRUM_MAX_SHELLS; b++) ac[b] = as[b] = 0.0;
   for (int64_t t0 = p0; t0 < p1; t0 += kSpecTile) {
     const int m = (int)(p1 - t0 < kSpecTile ? p1 - t0 : kSpecTile);
     __syncthreads();
@@ -176,25 +196,52 @@ __global__ void __launch_bounds__(256) k_spectrum(const double* __restrict__ X, 
       pz[i] = Z[t0 + i];
     }
     __syncthreads();
-    for (int i = 0; i < m; i++) {
-      const double x = px[i], y = py[i], z = pz[i];
+    for (int i = sub; i < m; i += 256 / kSpecDirs) {
+      // sum(k .* x) = (kx x + ky y) + kz z
+      const double kd = __dadd_rn(__dadd_rn(__dmul_rn(kx, px[i]), __dmul_rn(ky, py[i])), __dmul_rn(kz, pz[i]));
+      double s1, c1;
+      sincos(kd, &s1, &c1);
+      double ca = 0.0, sa = 0.0, cb = c1, sb = s1;  // the factors of the last two shells
 #pragma unroll
-      for (int j = 0; j < kSpecPairs; j++) {
-        // sum(k .* x) = (kx x + ky y) + kz z
-        const double kd = __dadd_rn(__dadd_rn(__dmul_rn(kx[j], x), __dmul_rn(ky[j], y)), __dmul_rn(kz[j], z));
-        double s, c;
-        sincos(kd, &s, &c);
-        ac[j] += c;
-        as[j] += s;
+      for (int b = 0; b < LCS_SPECTRUM_MAX_SHELLS; b++) {
+        if (b >= nshells) break;
+        double c = c1, s = s1;
+        if (b == 1) {
+          c = c1 * c1 - s1 * s1;
+          s = 2.0 * (c1 * s1);
+        } else if (b == 2) {
+          c = cb * c1 - sb * s1;
+          s = sb * c1 + cb * s1;
+        } else if (b > 2) {
+          c = ca * ca - sa * sa;
+          s = 2.0 * (ca * sa);
+        }
+        ac[b] += c;
+        as[b] += s;
+        ca = cb;
+        sa = sb;
+        cb = c;
+        sb = s;
       }
     }
   }
 #pragma unroll
-  for (int j = 0; j < kSpecPairs; j++)
-    if (pr[j] < npairs) {
-      partials[((int64_t)blockIdx.x * npairs + pr[j]) * 2] = ac[j];
-      partials[((int64_t)blockIdx.x * npairs + pr[j]) * 2 + 1] = as[j];
+  for (int b = 0; b < LCS_SPECTRUM_MAX_SHELLS; b++) {
+    if (b >= nshells) break;
+    __syncthreads();
+    red[0][threadIdx.x] = ac[b];
+    red[1][threadIdx.x] = as[b];
+    __syncthreads();
+    if (sub == 0 && dir < ns) {
+      double* o = partials + ((int64_t)blockIdx.x * nshells * ns + (int64_t)b * ns + dir) * 2;
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        double v = red[w][threadIdx.x];
+        for (int u = 1; u < 256 / kSpecDirs; u++) v += red[w][threadIdx.x + u * kSpecDirs];
+        o[w] = v;
+      }
     }
+  }
 }
 
 __global__ void __launch_bounds__(256) k_spectrum_final(const double* __restrict__ partials, int nb, int npairs,

@@ -115,3 +115,45 @@ def test_particle_stat_large():
     # weight: non-integer wave vectors are not orthogonal to the constant)
     assert st["spectrum"]["Enp"].size == 14 and np.all(np.isfinite(st["spectrum"]["Enp"]))
     g.close()
+
+
+@pytest.mark.parametrize("ns,max_wavenumber", [(2, 1), (64, 3), (65, 24), (200, 768)])
+def test_spectrum_shells_and_directions(ns, max_wavenumber):
+    """Every shell's phase factor is a product of wavenumber 1's; directions go
+    64 a block: one shell, the three that the rest build on, all 19, and a
+    partial block of directions.  The bound is the shot-noise one above; a phase
+    of 768 x 11 rad is rounded at 1e-12, far below it."""
+    cfg = make_config(16, species=[{"n": 700, "density_ratio": 843.0}], Re=50.0)
+    out = []
+    for cls in (Engine, OracleEngine):
+        e = cls(cfg)
+        rng = np.random.default_rng(5)
+        x, y, z = (rng.random(700) * 2 * np.pi for _ in range(3))
+        zero = np.zeros(700)
+        e.upload_particles(0, np.full(700, 0.02), x, y, z, zero, zero, zero, ids=np.arange(1, 701))
+        out.append(e.particles_stat(0, 1.0, nsamples=ns, max_wavenumber=max_wavenumber)["spectrum"])
+        e.close()
+    a, b = out
+    assert np.array_equal(a["wavenumbers"], b["wavenumbers"])
+    scale = 4 * np.pi * b["wavenumbers"] ** 2 / 700
+    assert np.all(np.abs(a["Enp"] - b["Enp"]) <= 1e-9 * scale)
+
+
+@pytest.mark.parametrize("span", [1.0, 1.4])
+@pytest.mark.parametrize("tol,radius,cells", [(0.01, 1e-3, 1), (0.5, 1e-2, 3), (4.0, 1e-3, 2)])
+def test_rdf_reach(span, tol, radius, cells):
+    """Counts where the contact distance lies beyond the last bin edge and
+    where particles lie outside the box (no cell is skipped then): exact."""
+    cfg = make_config(32, species=[{"n": 3000, "density_ratio": 843.0}], Re=50.0)
+    out = []
+    for cls in (Engine, OracleEngine):
+        e = cls(cfg)
+        rng = np.random.default_rng(9)
+        x, y, z = (rng.random(3000) * 2 * np.pi * span for _ in range(3))
+        zero = np.zeros(3000)
+        e.upload_particles(0, np.full(3000, 0.125), x, y, z, zero, zero, zero, ids=np.arange(1, 3001))
+        out.append(e.particles_stat(0, 1.0, search_cell_size=cells, contact_tolerance=tol, min_radius=radius,
+                                    max_wavenumber=1, nsamples=2)["rdf"])
+        e.close()
+    a, b = out
+    assert np.array_equal(a["npairs"], b["npairs"]) and a["npairs_contact"] == b["npairs_contact"]
