@@ -327,6 +327,7 @@ class Engine : public EngineBase {
   // order's bits, and a step is a few milliseconds either way.
   bool pot_ok = false;
   int debug_kind = 0;
+  int pot_tile = -1;  // LCS_B200_POT_TILE = 0, 1 or 2 (tests and timing): that tile of the sweep
   bool use_pot() const { return pot_ok && debug_kind == 0; }
     // Tiles of the sweep (warps x rows a warp).  Taller tiles do less redundant
   // work, a plane of shorter ones takes less time, and a grid of few tiles
@@ -356,6 +357,7 @@ class Engine : public EngineBase {
     LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotWS, kPotRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotS::bytes));
     LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotV::bytes));
     LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
+    if (const char* t = std::getenv("LCS_B200_POT_TILE")) pot_tile = std::max(0, std::min(2, std::atoi(t)));
     pot_ptrs.ctx[0] = dctx;
     pot_ptrs.P[0] = P;
     pot_ptrs.scratch[0] = (T*)stage;
@@ -376,9 +378,8 @@ class Engine : public EngineBase {
     const int rows[3] = {PotT::TY, PotS::TY, PotV::TY};
     const double plane_us[3] = {sizeof(T) == 8 ? 2.1 : 2.2, sizeof(T) == 8 ? 2.1 : 1.5, sizeof(T) == 8 ? 1.15 : 0.92};
     double best = 1e300;
-    const char* force = std::getenv("LCS_B200_POT_TILE");  // 0, 1 or 2 (the tests and timing): that tile
     for (int kind = 0; kind < 3; kind++) {
-      if (force && std::atoi(force) != kind) continue;
+      if (pot_tile >= 0 && pot_tile != kind) continue;
       const int gy = (g.n[1] + 1 + rows[kind] - 1) / rows[kind], cols = pg.gx * gy;
       for (int nc = std::max(cu > 0 ? (nu + cu - 1) / cu : 1, (2 * nu + kPotMaxChunk - 1) / kPotMaxChunk); nc <= nu; nc++) {
         const double cost = std::ceil((double)cols * nc / slots) * (2.0 * ((nu + nc - 1) / nc) + 12.0) * plane_us[kind];

@@ -145,7 +145,7 @@ __device__ __forceinline__ double pot_ulp2(float v) {
 __device__ __forceinline__ double pot_ulp2(double) { return 0.0; }
 
 // Start of a couple: D = div U (periodic, in FP64, rounded once), Phi = 0, J = 0.
-// Bound by HBM: 3 fields read, 2 written.
+// Bound by HBM: 3 fields read, 2 written (512^3: FP64 1.2 ms, 4.5 TB/s).
 //
 // FP32: the velocity is rounded to FP32 when it is stored, and that rounding
 // has a divergence of its own, which the sweeps of the velocity saw and the
@@ -223,7 +223,8 @@ __global__ void __launch_bounds__(256) k_pot_setup(const __grid_constant__ PotGr
 
 // The last group's jumps into J and D (nothing when it has none pending: the
 // first group, and a group that is run again).  One thread per face cell; the
-// cells of two faces belong to the z face, so each D is written once.
+// cells of two faces belong to the z face, so each D is written once.  Bound by
+// its launch (3 us up to 256^3, 10 at 512^3).
 template <typename T>
 __global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGroup<T> ga, PotGeom pg) {
   const int m = blockIdx.y;
@@ -304,8 +305,9 @@ __global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGro
 // of the core, then of the z slabs, the y slabs and the x slabs, as far as the
 // block's columns and its axis need them.  Blocks at the rim of a y or x slab
 // so sweep the few cells of the earlier slabs beside it themselves, and no
-// block waits for another: one launch instead of three (at 96^3 in FP32 the
-// three took 3 x 8 us).  A value reaches at most 5 columns (both colours of the
+// block waits for another: one launch instead of three (a step at 96^3 in FP32
+// 13.4 -> 10.4 ms, 512^3 as before).  Bound by the latency of its loads and its
+// four to eight phases (11 us up to 128^3).  A value reaches at most 5 columns (both colours of the
 // x, the y and the z slab, where the y slab crosses to the z slab in place),
 // so 22 x 22 of the columns are the block's own.
 template <typename T, int AX>
@@ -508,6 +510,14 @@ struct PotLoop {
 // With overlap, k_pot_slab has put the first sweep's values into the halo and
 // the outer layers; without, the halo is the periodic image, read in place
 // (pairs never straddle the period: n is even).
+//
+// A group at 512^3: FP32 1.05 ms (12 x 4 rows), FP64 1.8 ms (8 x 4), where the
+// three element-wise sweeps with their slabs and fill took 3.7 and 6.2; at the
+// HBM peak its 3 values a cell take 0.25 and 0.49.  It is bound by instruction
+// issue and latency: issue 54 % (FP32) and 37 % (FP64) of the cycles, DRAM 29
+// and 35 %, the shared-memory pipe 41 and 53 %.  The tile is as tall as the
+// registers allow (168 and 254 a thread): a row's two colours at 7 planes live
+// in them, and D, read once in three half sweeps each, in shared memory.
 template <typename T, int NW, int RW>
 __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
     k_pot_sweep(const __grid_constant__ PotGroup<T> ga, PotGeom pg, HsmacCoef cf, PotLoop loop) {
@@ -801,7 +811,7 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
 }
 
 // End of a couple: the velocity and P from Phi.  Bound by HBM: 5 fields read,
-// 4 written.
+// 4 written (512^3: FP64 2.1 ms, FP32 1.03: 4.6 TB/s).
 template <typename T>
 __global__ void __launch_bounds__(256) k_pot_apply(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg) {
   const int m = blockIdx.y;
