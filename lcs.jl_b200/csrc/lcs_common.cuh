@@ -146,4 +146,7 @@ __host__ __device__ __forceinline__ int wrap1(int i, int n) {
   return (r < 0 ? r + n : r) + 1;
 }
 
+// the same for 1-n..2n (no division)
+__host__ __device__ __forceinline__ int wrap_near(int i, int n) { return i < 1 ? i + n : i > n ? i - n : i; }
+
 }  // namespace lcs
