@@ -109,7 +109,13 @@ struct Ctx {
   int pot_cur;      // which spare buffer holds the group's input potential
   int pot_pending;  // the last group's jumps are not yet in the right-hand side
   int pot_redo;     // sweeps of the group to run again (the exit lay inside it), 0: none
-  double pot_floor; // mean square divergence of the FP32 velocity's rounding (0 in FP64)
+  // FP32 only, see k_pot_jump: what the residual's sum has to have added for the
+  // rounding of the stored velocity (0: not measured in this couple),
+  // groups since it was measured, residual sums of the last group, and the
+  // state of exit tests that wait for it (1: to be measured, 2: tested, the
+  // rest of this group does nothing).
+  double pot_round, pot_sum[3];
+  int pot_age, pot_check;
 };
 
 // ---- stencil primitives (src/diff.jl:1-39), same evaluation order --------

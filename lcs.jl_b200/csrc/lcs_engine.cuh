@@ -408,6 +408,8 @@ class Engine : public EngineBase {
     pg.dxi = hc.dxi;
     pg.dyi = hc.dyi;
     pg.dzi = hc.dzi;
+    const double rms = hc.epsp / hc.dxmin;
+    pg.exit_sum = rms > 0.0 ? rms * rms * hc.count * (1.0 + 1e-12) : 0.0;
     return pg;
   }
   const PotGroup<T>& pot_args() const { return grp ? grp_pot : pot_ptrs; }
@@ -425,13 +427,24 @@ class Engine : public EngineBase {
     const int64_t half = (int64_t)g.n[0] / 2 * g.n[1] * g.n[2];
     return launch("pot_apply", k_pot_apply<T>, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
   }
+  // FP32: the rounding of the stored velocity into the logged residual
+  int pot_round(int set) {
+    if constexpr (sizeof(T) == 8) {
+      return LCS_OK;
+    } else {
+      const dim3 grid(blocks_for((int64_t)g.n[0] * g.n[1] * g.n[2], 256), pot_members());
+      return launch("pot_round", k_pot_round<T>, grid, dim3(256), 0, pot_args(), g, set, pot_geom(), hc);
+    }
+  }
   // one group of three sweeps
-  int pot_group(const PotLoop& loop) {
+  int pot_group(int set, const PotLoop& loop) {
     const PotGeom pg = pot_geom();
     const int M = pot_members();
     if (3 * (int64_t)pg.nseg + pg.nslab > plan.partials_cap) return fail(LCS_EINVAL, "grid too large for the partials buffer");
     const int64_t faces = (int64_t)g.n[0] * g.n[1] + (int64_t)g.n[0] * g.n[2] + (int64_t)g.n[1] * g.n[2];
-    LCS_TRY(launch("pot_jump", k_pot_jump<T>, dim3(blocks_for(faces, 256), M), dim3(256), 0, pot_args(), pg));
+    // (FP32: it has all cells to visit when it measures the velocity's rounding)
+    const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2], jump = sizeof(T) == 4 ? std::max(faces, cells / 4) : faces;
+    LCS_TRY(launch("pot_jump", k_pot_jump<T>, dim3(blocks_for(jump, 256), M), dim3(256), 0, pot_args(), g, set, pg, hc));
     if (cfg.overlap)
       LCS_TRY(launch("pot_slab", k_pot_slab<T>, dim3(pg.nslab, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg));
     const dim3 grid(pg.nseg, M);
@@ -928,7 +941,7 @@ class Engine : public EngineBase {
   }
   // One iteration of the reference's `while itr < itrmax` loop.
   int couple_group(int set) {
-    if (use_pot()) return pot_group(PotLoop{});
+    if (use_pot()) return pot_group(set, PotLoop{});
     const int n0 = g.n[0], h = g.h;
     (void)n0;
     const Box full = cube(g, 1 - h, h);
@@ -955,8 +968,12 @@ class Engine : public EngineBase {
   }
   int sweeps_per_group() const { return cfg.time_blocking ? 3 : 1; }
   // iterations of a couple's loop: at most ceil(itrmax / sweeps per group),
-  // plus a margin (the device loop and the host loop use the same bound)
-  int max_loop_groups() const { return cfg.itrmax / sweeps_per_group() + 2; }
+  // plus a margin (the device loop and the host loop use the same bound);
+  // twice that where a group's exit tests can take another one (k_pot_jump)
+  int max_loop_groups() const {
+    const int n = cfg.itrmax / sweeps_per_group() + 2;
+    return use_pot() && sizeof(T) == 4 ? 2 * n : n;
+  }
 
   int read_ctx() {
     LCS_TRY(copy(hctx, dctx, sizeof(Ctx), cudaMemcpyDeviceToHost));
@@ -977,7 +994,8 @@ class Engine : public EngineBase {
     // the device advances itr by one per sweep until it exits; the group
     // count is bounded so the host loop ends even if that ever failed
     const int max_groups = max_loop_groups();
-    bool again = false;  // the exit lay inside a potential-form group, which runs again up to it
+    // a potential-form group whose exit tests are still to run, or that runs again up to the exit inside it
+    bool again = false;
     for (int grp = 0; itr < cfg.itrmax || again; grp++) {
       if (grp >= max_groups) return fail(LCS_ETIMEDOUT, "HSMAC loop did not advance");
       LCS_TRY(couple_group(set));
@@ -988,12 +1006,15 @@ class Engine : public EngineBase {
         if (hctx->nonfinite) return fail(LCS_ENONFINITE, "HSMAC residual is not finite");
         if (hctx->cs.done) break;
         itr = hctx->cs.itr;
-        again = use_pot() && hctx->pot_redo != 0;
+        again = use_pot() && (hctx->pot_redo || hctx->pot_check);
       } else {
         itr += spg;
       }
     }
-    if (use_pot()) LCS_TRY(pot_apply(set));
+    if (use_pot()) {
+      LCS_TRY(pot_round(set));
+      LCS_TRY(pot_apply(set));
+    }
     return launch("couple_log", k_couple_log, dim3(1), dim3(1), 0, dctx, stage);
   }
 
@@ -1094,7 +1115,7 @@ class Engine : public EngineBase {
     stream = side;
     int rc2 = LCS_OK;
     if (use_pot()) {
-      for (int q = 0; q < pot_unroll() && rc2 == LCS_OK; q++) rc2 = pot_group(PotLoop{1, max_loop_groups(), handle});
+      for (int q = 0; q < pot_unroll() && rc2 == LCS_OK; q++) rc2 = pot_group(set, PotLoop{1, max_loop_groups(), handle});
     } else {
       rc2 = couple_group(set);
     }
@@ -1107,7 +1128,10 @@ class Engine : public EngineBase {
     if (rc2 != LCS_OK) return rc2;
     if (e != cudaSuccess) return fail(LCS_ECUDA, "capture of the couple loop: %s", cudaGetErrorString(e));
     LCS_CUDA(cudaStreamUpdateCaptureDependencies(stream, &node, 1, cudaStreamSetCaptureDependencies));
-    if (use_pot()) LCS_TRY(pot_apply(set));
+    if (use_pot()) {
+      LCS_TRY(pot_round(set));
+      LCS_TRY(pot_apply(set));
+    }
     return launch("couple_log", k_couple_log, dim3(1), dim3(1), 0, dctx, stage);
   }
 
@@ -2165,7 +2189,8 @@ struct EngineGroup : GroupBase {
     LCS_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
     if (L->use_pot()) {
       L->grp = &mem;
-      const int ra = L->pot_apply(set);
+      int ra = L->pot_round(set);
+      if (ra == LCS_OK) ra = L->pot_apply(set);
       L->grp = nullptr;
       LCS_GTRY(L, ra);
     }

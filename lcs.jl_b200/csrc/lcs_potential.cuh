@@ -120,6 +120,7 @@ struct PotGeom {
   int slab0[3];            // first tile of an axis's slabs (z, y, x in turn)
   double cx, cy, cz, k0, wd;  // 1/dx^2 .., 2 (cx + cy + cz), -omega dl
   double dxi, dyi, dzi;
+  double exit_sum;         // the exit test's bound on a sweep's sum of div^2 (a hair above it)
 };
 
 __device__ __forceinline__ int pot_wrap(int i, int n) {  // 1-based image of i in -n < i
@@ -137,26 +138,8 @@ template <typename T> __device__ __forceinline__ T* pot_rhs(const Ctx* ctx) { re
 __device__ __forceinline__ int pot_layer(int i, int nx) { return i <= 4 ? 2 + i : i >= nx - 2 ? i - (nx - 2) : -1; }
 __device__ __forceinline__ int pot_dlayer(int i, int nx) { return i <= 3 ? 1 + i : i >= nx - 1 ? i - (nx - 1) : -1; }
 
-// Square of the spacing of the FP32 numbers around v (0 for FP64, see below).
-__device__ __forceinline__ double pot_ulp2(float v) {
-  const double u = (double)__int_as_float(__float_as_int(v) & 0x7f800000) * (1.0 / 8388608.0);
-  return u * u;
-}
-__device__ __forceinline__ double pot_ulp2(double) { return 0.0; }
-
 // Start of a couple: D = div U (periodic, in FP64, rounded once), Phi = 0, J = 0.
 // Bound by HBM: 3 fields read, 2 written (512^3: FP64 1.2 ms, 4.5 TB/s).
-//
-// FP32: the velocity is rounded to FP32 when it is stored, and that rounding
-// has a divergence of its own, which the sweeps of the velocity saw and the
-// potential does not.  The exit test is on the divergence of the velocity, so
-// the residual of every sweep includes it: each of a cell's six faces is
-// rounded with variance ulp^2 / 12, which gives the sum over the faces of
-// ulp^2 / 12 / da^2 per cell (3.2e-7, 6.3e-7 and 1.26e-6 rms at 32^3, 64^3 and
-// 128^3; the stored velocity's divergence is 3.3e-7, 6.4e-7 and 1.28e-6, and
-// sweeping the velocity itself to the end leaves 2.5e-7, 5.9e-7 and 1.5e-6).
-// Without it FP32 couples at 32^3 left the loop after 250 sweeps, at a
-// residual of 1e-8 that the FP32 velocity does not have.
 template <typename T>
 __global__ void __launch_bounds__(256) k_pot_setup(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg) {
   const int m = blockIdx.y;
@@ -170,18 +153,11 @@ __global__ void __launch_bounds__(256) k_pot_setup(const __grid_constant__ PotGr
   const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const int hx = nx / 2;
   const int total = hx * ny * nz;  // < 2^31 (host)
-  __shared__ double red[8];
-  __shared__ int last;
-  double q2 = 0.0;
   for (int t = blockIdx.x * 256 + threadIdx.x; t < total; t += gridDim.x * 256) {
     const int i = 1 + 2 * (t % hx);
     const int u = t / hx;
     const int j = 1 + u % ny, k = 1 + u / ny;
     const int64_t c = g.at(i, j, k);
-    // (every face belongs to two cells)
-    if (sizeof(T) == 4)
-      q2 += (pg.cx * (pot_ulp2(U[c]) + pot_ulp2(U[c + 1])) + pg.cy * (pot_ulp2(V[c]) + pot_ulp2(V[c + 1])) +
-             pg.cz * (pot_ulp2(W[c]) + pot_ulp2(W[c + 1]))) * (2.0 / 12.0);
     const int64_t cw = i > 1 ? c - 1 : g.at(nx, j, k);
     const int64_t cs = j > 1 ? c - g.px : g.at(i, ny, k);
     const int64_t cb = k > 1 ? c - g.pz : g.at(i, j, nz);
@@ -206,30 +182,162 @@ __global__ void __launch_bounds__(256) k_pot_setup(const __grid_constant__ PotGr
     ctx->pot_cur = 0;
     ctx->pot_pending = 0;
     ctx->pot_redo = 0;
-    if (sizeof(T) == 8) ctx->pot_floor = 0.0;
+    ctx->pot_round = 0.0;
+    ctx->pot_age = 0;
+    ctx->pot_check = 0;
   }
-  if (sizeof(T) == 4) {
-    const double b = block_sum<256>(q2, red);
-    if (threadIdx.x == 0) ga.partials[m][blockIdx.x] = b;
-    if (last_block(&ctx->ticket, gridDim.x, &last)) {
-      const double sum = sum_partials<256>(ga.partials[m], (int)gridDim.x, red);
-      if (threadIdx.x == 0) {
-        ctx->pot_floor = sum / ((double)nx * ny * nz);
-        ctx->ticket = 0;
-      }
+}
+
+// The exit tests of a group's three sweeps, from their sums of div^2 (FP32:
+// each with `round`, that of the stored velocity).  The state of the loop and
+// of the potential after them.
+__device__ __forceinline__ void pot_exit(Ctx* ctx, const HsmacCoef& cf, const double sum[3], double round) {
+  int again = 0;  // the exit lies inside the group: run it again up to that sweep
+  for (int q = 0; q < 3; q++) {
+    hsmac_check(ctx, cf, sum[q] + round, 1);
+    if (ctx->cs.done) {
+      if (q < 2 && isfinite(ctx->cs.div)) again = q + 1;
+      break;
     }
   }
+  if (again) {
+    ctx->cs.done = 0;
+    ctx->cs.cont = 1;
+  }
+  ctx->pot_redo = again;
+  ctx->pot_pending = again ? 0 : 1;
+  if (!again) ctx->pot_cur = 1 - ctx->pot_cur;
+}
+
+// FP32: this block's share of the sum over the cells of e^2, where e is the
+// divergence of the velocity as it would be stored for the potential `phi` (a
+// group's output, its jumps pending) less the divergence that the sweeps see
+// there.  It holds every rounding between the two: of the velocity's faces, of
+// D and of the sweeps' own sums.  Bound by the latency of its 14 loads a cell.
+template <typename T>
+__device__ __forceinline__ double pot_round_sum(const Ctx* ctx, const Grid& g, int set, const T* __restrict__ phi,
+                                                const T* __restrict__ s, const PotGeom& pg) {
+  const T* __restrict__ U = (const T*)ctx->vel[set][0];
+  const T* __restrict__ V = (const T*)ctx->vel[set][1];
+  const T* __restrict__ W = (const T*)ctx->vel[set][2];
+  const T* __restrict__ D = pot_rhs<T>(ctx);
+  const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz, px = pg.s.px, pz = pg.s.pz;
+  const T cx = (T)pg.cx, cy = (T)pg.cy, cz = (T)pg.cz, k0 = (T)pg.k0;
+  double acc = 0.0;
+  const int total = nx * ny * nz;  // < 2^31 (host)
+  for (int64_t t64 = (int64_t)blockIdx.x * 256 + threadIdx.x; t64 < total; t64 += (int64_t)gridDim.x * 256) {
+    const int t = (int)t64;
+    const int i = 1 + t % nx, r = t / nx, j = 1 + r % ny, k = 1 + r / ny;
+    const int o = pg.s.at(i, j, k);
+    const int64_t c = g.at(i, j, k);
+    const T p = phi[o];
+    // of an axis: the divergence of the two faces as stored, and the sum of
+    // the two neighbours as the sweeps see them.  lo, hi: the neighbours'
+    // images; a, b: the low and the high face's velocity; (first, last): the
+    // cell lies there, f: its place on the face.
+    auto axis = [&](int ax, T lo, T hi, T a, T b, bool first, bool last, int f, double di, T* nsum) {
+      T vlo = p, vhi = hi;  // the high neighbour of the low face's cell, and of this one, as k_pot_apply has them
+      T slo = lo, shi = hi;
+      if (first || last) {
+        const T e = s[pg.s.e[ax] + f], head = first ? p : hi;  // Phi(1)
+        const T jmp = s[pg.s.j[ax] + f] + (head - e);
+        if (first) {
+          vlo = head - jmp;
+          slo = lo + (head - e);
+        }
+        if (last) {
+          vhi = head - jmp;
+          shi = e;
+        }
+      }
+      *nsum = slo + shi;
+      const T d = (T)di;
+      return di * ((double)pfma<T>(d, p - vhi, b) - (double)pfma<T>(d, lo - vlo, a));
+    };
+    const bool x1 = i == 1, xn = i == nx, y1 = j == 1, yn = j == ny, z1 = k == 1, zn = k == nz;
+    const int fx = (k - 1) * ny + (j - 1), fy = (k - 1) * nx + (i - 1), fz = (j - 1) * nx + (i - 1);
+    T sx, sy, sz;
+    double div = axis(0, phi[x1 ? o + (nx - 1) : o - 1], phi[xn ? o - (nx - 1) : o + 1],
+                      U[x1 ? c + (nx - 1) : c - 1], U[c], x1, xn, fx, pg.dxi, &sx);
+    div += axis(1, phi[y1 ? o + (ny - 1) * px : o - px], phi[yn ? o - (ny - 1) * px : o + px],
+                V[y1 ? g.at(i, ny, k) : c - g.px], V[c], y1, yn, fy, pg.dyi, &sy);
+    div += axis(2, phi[z1 ? o + (nz - 1) * pz : o - pz], phi[zn ? o - (nz - 1) * pz : o + pz],
+                W[z1 ? g.at(i, j, nz) : c - g.pz], W[c], z1, zn, fz, pg.dzi, &sz);
+    T d = D[o];  // (without the x jumps so far)
+    if (x1) d -= cx * s[pg.s.j[0] + fx];
+    if (xn) d += cx * s[pg.s.j[0] + fx];
+    const double e = div - (double)pot_div<T>(p, sx, sy, sz, d, cx, cy, cz, k0);
+    acc += e * e;
+  }
+  return acc;
+}
+
+// FP32, after a couple that ran to its last sweep: the rounding of the stored
+// velocity into the residual that the log shows (a couple that left by the exit
+// test has it: k_pot_jump).  12 us at 32^3, 240 at 256^3, 1.8 ms at 512^3.
+template <typename T>
+__global__ void __launch_bounds__(256) k_pot_round(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg,
+                                                   HsmacCoef cf) {
+  __shared__ double red[8];
+  __shared__ int last;
+  const int m = blockIdx.y;
+  Ctx* ctx = ga.ctx[m];
+  if (ctx->cs.done || !ctx->pot_pending) return;
+  const double acc = pot_round_sum<T>(ctx, g, set, pot_buf<T>(ctx, ctx->pot_cur), ga.scratch[m], pg);
+  const double b = block_sum<256>(acc, red);
+  if (threadIdx.x == 0) ga.partials[m][blockIdx.x] = b;
+  if (!last_block(&ctx->ticket, gridDim.x, &last)) return;
+  const double sum = sum_partials<256>(ga.partials[m], (int)gridDim.x, red);
+  if (threadIdx.x != 0) return;
+  ctx->ticket = 0;
+  ctx->pot_round = sum * (cf.count / ((double)pg.s.nx * pg.s.ny * pg.s.nz));
+  ctx->cs.sum = ctx->pot_sum[2] + ctx->pot_round;
+  ctx->cs.div = sqrt(ctx->cs.sum / cf.count);
 }
 
 // The last group's jumps into J and D (nothing when it has none pending: the
 // first group, and a group that is run again).  One thread per face cell; the
 // cells of two faces belong to the z face, so each D is written once.  Bound by
 // its launch (3 us up to 256^3, 10 at 512^3).
+//
+// FP32: the exit test is on the divergence of the velocity, which is stored in
+// FP32, and that rounding has a divergence of its own that the potential does
+// not show (u_rms 1: 3.3e-7, 6.4e-7 and 1.28e-6 rms at 32^3, 64^3 and 128^3).
+// So when a sweep's own residual would let the couple end, its group's tests
+// wait (pot_check = 1): this kernel, the first of the next group, measures the
+// rounding at the group's output (pot_round_sum) and its last block runs the
+// tests, and that group does nothing else (pot_check = 2 until its sweep ends).
+// A measurement holds for the groups after it while it keeps the residual above
+// the exit by a factor of two in the square, for at most kPotRoundAge of them
+// (a couple at 32^3 passes an exit of 1e-8 after 250 sweeps and goes on to 300:
+// two measurements, 20 us each; after every eighth group they took 8 % of a step).
+constexpr int kPotRoundAge = 32;
 template <typename T>
-__global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGroup<T> ga, PotGeom pg) {
+__global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg,
+                                                  HsmacCoef cf) {
   const int m = blockIdx.y;
   Ctx* ctx = ga.ctx[m];
-  if (ctx->cs.done || !ctx->cs.cont || !ctx->pot_pending) return;
+  const int done = ctx->cs.done, cont = ctx->cs.cont, pending = ctx->pot_pending, check = ctx->pot_check;  // one latency
+  if (done || !cont) return;
+  if constexpr (sizeof(T) == 4) {
+    if (check) {
+      __shared__ double red[8];
+      __shared__ int last;
+      const double acc = pot_round_sum<T>(ctx, g, set, pot_buf<T>(ctx, 1 - ctx->pot_cur), ga.scratch[m], pg);
+      const double b = block_sum<256>(acc, red);
+      if (threadIdx.x == 0) ga.partials[m][blockIdx.x] = b;
+      if (!last_block(&ctx->ticket, gridDim.x, &last)) return;
+      const double sum = sum_partials<256>(ga.partials[m], (int)gridDim.x, red);
+      if (threadIdx.x != 0) return;
+      ctx->ticket = 0;
+      ctx->pot_round = sum * (cf.count / ((double)pg.s.nx * pg.s.ny * pg.s.nz));
+      ctx->pot_age = 0;
+      pot_exit(ctx, cf, ctx->pot_sum, ctx->pot_round);
+      ctx->pot_check = 2;
+      return;
+    }
+  }
+  if (!pending) return;
   const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz;
   T* D = pot_rhs<T>(ctx);
   T* s = ga.scratch[m];
@@ -456,7 +564,8 @@ __global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_const
   const int m = blockIdx.y, b = blockIdx.x;
   const Ctx* ctx = ga.ctx[m];
   // (a group that runs again finds these in place)
-  if (ctx->cs.done || !ctx->cs.cont || ctx->pot_redo) return;
+  const int done = ctx->cs.done, cont = ctx->cs.cont, redo = ctx->pot_redo, check = ctx->pot_check;
+  if (done || !cont || redo || check) return;
   T* sh = (T*)smem_raw;  // [10][32][32]
   if (b < pg.slab0[1]) pot_slab_body<T, 2>(ga, pg, m, b, sh, red);
   else if (b < pg.slab0[0]) pot_slab_body<T, 1>(ga, pg, m, b - pg.slab0[1], sh, red);
@@ -533,8 +642,18 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   int* sZ = (int*)((T*)smem_raw + L::d_elems + L::x_elems);  // box bits of the planes kb - 13 ..
   const int m = blockIdx.y;
   Ctx* ctx = ga.ctx[m];
-  if (ctx->cs.done || !ctx->cs.cont) return;
-  const int cur = ctx->pot_cur, redo = ctx->pot_redo;
+  const int done = ctx->cs.done, cont = ctx->cs.cont, cur = ctx->pot_cur, redo = ctx->pot_redo, check = ctx->pot_check;
+  if constexpr (sizeof(T) == 4) {
+    if (check) {  // this group ran the last one's exit tests (k_pot_jump); they may have ended the couple
+      if (last_block(&ctx->ticket, gridDim.x, &last_flag) && threadIdx.x == 0) {
+        ctx->ticket = 0;
+        ctx->pot_check = 0;
+        if (loop.on) cudaGraphSetConditional(loop.handle, couple_goes_on(ctx, loop.max_groups) ? 1u : 0u);
+      }
+      return;
+    }
+  }
+  if (done || !cont) return;
   const int nsw = redo ? redo : 3;  // sweeps of this pass
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz;
@@ -776,6 +895,8 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
     if (tid == 0) part[3 * blockIdx.x + q] = bs;
   }
   if (!last_block(&ctx->ticket, nb, &last_flag)) return;
+  const double round = sizeof(T) == 4 ? ctx->pot_round : 0.0;
+  const int itr = ctx->cs.itr, age = ctx->pot_age + 1;
   double sum[3];
 #pragma unroll
   for (int q = 0; q < 3; q++) {
@@ -787,26 +908,27 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   }
   if (tid != 0) return;
   ctx->ticket = 0;
-  int again = 0;  // the exit lies inside the group: run it again up to that sweep
-  if (redo == 0) {
-    for (int q = 0; q < 3; q++) {
-      hsmac_check(ctx, cf, sum[q] + ctx->pot_floor * cf.count, 1);
-      if (ctx->cs.done) {
-        if (q < 2 && isfinite(ctx->cs.div)) again = q + 1;
-        break;
-      }
-    }
-    if (again) {
-      ctx->cs.done = 0;
-      ctx->cs.cont = 1;
-    }
-  } else {
+  if (redo) {
     ctx->cs.done = 1;
     ctx->cs.cont = 0;
+    ctx->pot_redo = 0;
+    ctx->pot_pending = 1;
+    ctx->pot_cur = 1 - cur;
+  } else {
+    bool wait = false;
+    if constexpr (sizeof(T) == 4) {
+      for (int q = 0; q < 3; q++)
+        if (itr + q >= cf.itrmin &&
+            (sum[q] + 0.5 * round <= pg.exit_sum || (sum[q] <= pg.exit_sum && age >= kPotRoundAge)))
+          wait = true;
+      wait = wait && isfinite(sum[0] + sum[1] + sum[2]);
+      if (wait || itr + 3 >= cf.itrmax)  // (k_pot_jump or k_pot_round adds the rounding to them)
+        for (int q = 0; q < 3; q++) ctx->pot_sum[q] = sum[q];
+      if (round > 0.0) ctx->pot_age = age;
+    }
+    if (wait) ctx->pot_check = 1;
+    else pot_exit(ctx, cf, sum, round);
   }
-  ctx->pot_redo = again;
-  ctx->pot_pending = again ? 0 : 1;
-  if (!again) ctx->pot_cur = 1 - cur;
   if (loop.on) cudaGraphSetConditional(loop.handle, couple_goes_on(ctx, loop.max_groups) ? 1u : 0u);
 }
 

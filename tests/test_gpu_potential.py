@@ -119,3 +119,91 @@ def test_group_equals_members_alone(precision):
     from lcs_b200 import _abi as abi
 
     serve_cases.check_group_equals_members_alone(Engine, abi.load_library(), precision, count=5, nsteps=2, n=28)
+
+
+@pytest.mark.parametrize("n", [8, 32, 54])
+def test_fp32_uniform_flow_leaves_at_itrmin(n):
+    """A uniform flow is free of divergence in FP32 too: residual 0, the exit
+    and the counts of the oracle."""
+    out = []
+    for cls in (Engine, OracleEngine):
+        e = cls(make_config(n, mode=F.MODE_FLOW, itrmin=7, itrmax=60, epsp=1e-8 * 2 * np.pi / n,
+                            precision=F.PRECISION_FP32_MIXED))
+        for f, v in ((0, 1.0), (1, -0.3), (2, 0.1), (6, 0.0)):
+            e.field_set(f, np.full(e.interior_shape, v))
+        out.append(e.couple(2, 0.004))
+        e.close()
+    assert out[0] == out[1] and out[0]["itr"] == 7 and out[0]["div"] == 0.0
+
+
+def smooth(shape, rng):
+    """U, V, W of 24 Fourier modes each (|k| <= 3 an axis, rms about 0.5) without
+    divergence, and a thousandth of it with: what a time step hands to a couple."""
+    nz, ny, nx = shape
+    pts = np.meshgrid(*(np.arange(m) * (2 * np.pi / m) for m in (nz, ny, nx)), indexing="ij")[::-1]
+    out = []
+    for a in range(3):
+        f = np.zeros(shape)
+        for _ in range(24):
+            k = rng.integers(-3, 4, 3)
+            amp = 0.15 if rng.random() < 0.5 else 1.5e-4
+            if amp > 0.1:
+                k[a] = 0
+            f += amp * np.sin(sum(k[b] * pts[b] for b in range(3)) + rng.random() * 6.3)
+        out.append(f)
+    return out
+
+
+@pytest.mark.parametrize("ov", [True, False])
+@pytest.mark.parametrize("n", [24, 32, 48])
+def test_fp32_residual_is_the_stored_velocitys(n, ov):
+    """Long FP32 couples.  Rounding the stored faces (about 0.5, 1.2e-8 rms)
+    leaves a divergence of sqrt(6) 1.2e-8 / dx = 1.1e-7 to 2.2e-7; the sweeps
+    relax Phi (5e-4) until its own rounding stops them, below 1e-8.  So with an
+    exit at 4e-8 the couple must not leave, although the potential alone would,
+    and the logged residual is the stored velocity's divergence up to twice
+    1e-8, 15 % of the former."""
+    e = Engine(make_config(n, mode=F.MODE_FLOW, overlap=ov, itrmin=6, itrmax=900, epsp=4e-8 * 2 * np.pi / n,
+                           precision=F.PRECISION_FP32_MIXED))
+    for f, a in enumerate(smooth(e.interior_shape, np.random.default_rng(n))):
+        e.field_set(f, a)
+    lg = e.couple(2, 0.004)
+    rms, _ = e.flow_divergence()
+    e.close()
+    assert lg["itr"] == lg["sweeps"] == 900
+    assert abs(lg["div"] - rms) <= 0.15 * rms, (lg, rms)
+
+
+@pytest.mark.parametrize("itrmin", [6, 7, 8])
+@pytest.mark.parametrize("epsp", [1e3, 3e-3])
+@pytest.mark.parametrize("ov", [True, False])
+def test_fp32_exit_equals_the_oracles(itrmin, epsp, ov):
+    """Exits after each sweep of a group, and on the residual far above the
+    rounding: the oracle's counts (a residual falls by 1 % or more a sweep, FP32
+    changes it by 1e-6)."""
+    dims = (40, 24, 32)
+    lg, g = couple(Engine, dims, ov, itrmin, 200, epsp, F.PRECISION_FP32_MIXED)
+    lo, o = couple(OracleEngine, dims, ov, itrmin, 200, epsp)
+    assert lg["itr"] == lo["itr"] < 200 and lg["sweeps"] == lo["sweeps"]
+    for a, b in zip(g[:3], o[:3]):
+        assert rel_l2(a, b) <= 1e-5
+
+
+@pytest.mark.parametrize("rms,itrmax", [(3e-8, 420), (1e-4, 420)])
+def test_fp32_step_graph_equals_direct_calls(rms, itrmax):
+    """The device-side loop in FP32: with the rounding measured and above the
+    exit (3e-8), and with an exit (1e-4)."""
+    out = []
+    for graphs in (0, 1):
+        e = Engine(make_config(32, mode=F.MODE_FLOW, Re=50.0, itrmin=6, itrmax=itrmax, epsp=rms * 2 * np.pi / 32,
+                               graphs=graphs, precision=F.PRECISION_FP32_MIXED))
+        e.upload_flow(*smooth(e.interior_shape, np.random.default_rng(4)), np.zeros(e.interior_shape))
+        logs = e.step(2)
+        out.append((logs, e.download_flow()))
+        e.close()
+    (la, fa), (lb, fb) = out
+    for x, y in zip(la, lb):
+        assert x["couple1"] == y["couple1"] and x["couple2"] == y["couple2"]
+        assert (x["couple2"]["itr"] == itrmax) == (rms < 1e-7)
+    for a, b in zip(fa, fb):
+        assert np.array_equal(a, b)
