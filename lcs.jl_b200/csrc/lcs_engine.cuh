@@ -403,7 +403,6 @@ class Engine : public EngineBase {
     pg.cx = hc.dxi * hc.dxi;
     pg.cy = hc.dyi * hc.dyi;
     pg.cz = hc.dzi * hc.dzi;
-    pg.k0 = 2.0 * (pg.cx + pg.cy + pg.cz);
     pg.wd = -hc.omega * hc.dl;
     pg.dxi = hc.dxi;
     pg.dyi = hc.dyi;
