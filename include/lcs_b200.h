@@ -203,7 +203,17 @@ LCS_API int lcs_flow_rhs(lcs_handle* h, int32_t stage);
 LCS_API int lcs_flow_update(lcs_handle* h, int32_t stage, double dtrk);
 /* rhs! then update! fused in one pass (dUdts is not written). */
 LCS_API int lcs_flow_rhs_update(lcs_handle* h, int32_t stage, double dtrk);
-/* `Flows.couple!(::HSMAC)` (src/flows/couples/hsmac.jl:52-75) on Us_couple(stage). */
+/* `Flows.couple!(::HSMAC)` (src/flows/couples/hsmac.jl:52-75) on Us_couple(stage).
+ * Time-blocked red-black-fast couples run in potential form (except FP64 grids
+ * of up to 40^3 cells, and where LCS_B200_FUSED_SWEEP is rw or plain or one of
+ * LCS_B200_RW, LCS_B200_FACES and LCS_B200_ZCHUNK is set: those select the
+ * element-wise sweeps): cells are visited in the reference's order and the
+ * sweep counts are its, the fields equal the element-wise sweeps' to rounding
+ * (FP64 1e-14, FP32 1e-5, P 1e-3) and not bit for bit.  FP32: the residual is
+ * that of the sweeps with the divergence that rounding leaves in the stored
+ * velocity.  The halos of U, V, W and P are the images of the interior
+ * afterwards; element-wise sweeps leave them as the reference's do, near that
+ * until the next synchalo. */
 LCS_API int lcs_flow_couple(lcs_handle* h, int32_t stage, double dtrk, lcs_couple_log* log);
 /* `Flows.forcing!` stage 2 (src/flows/forcings/{lf,rcf}.jl) on Us; p and e10 out. */
 LCS_API int lcs_flow_forcing(lcs_handle* h, double dtrk, double* p, double* e10);

@@ -228,3 +228,20 @@ def test_fp64_error_of_long_couples(n):
         e.close()
     errs = [rel_l2(a, b) for a, b in zip(*out)]
     assert max(errs) <= 4e-15, errs
+
+
+@pytest.mark.parametrize("precision", [F.PRECISION_FP64, F.PRECISION_FP32_MIXED])
+@pytest.mark.parametrize("dims,h,ov", [((24, 26, 30), 3, True), ((8, 8, 8), 3, True), ((10, 32, 8), 5, False)])
+def test_halos_after_a_couple(dims, h, ov, precision):
+    """The halos of U, V, W and P are the images of the interior, whatever they
+    held: exactly."""
+    e = Engine(make_config(dims=dims, h=h, mode=F.MODE_FLOW, overlap=ov, itrmin=6, itrmax=9, epsp=1e-12,
+                           precision=precision))
+    rng = np.random.default_rng(2)
+    for f in (0, 1, 2, 6):
+        e.field_set(f, rng.standard_normal(e.haloed_shape), haloed=True)
+    e.couple(2, 0.004)
+    for f in (0, 1, 2, 6):
+        a = e.field_get(f, haloed=True)
+        assert np.array_equal(a, np.pad(a[h:-h, h:-h, h:-h], h, mode="wrap")), f
+    e.close()
