@@ -2172,10 +2172,12 @@ struct EngineGroup : GroupBase {
     if (rc2 == LCS_OK) {
       L->stream = side;
       L->grp = &mem;
-      for (int q = 0; q < (L->use_pot() ? L->pot_unroll() : 1) && rc2 == LCS_OK; q++) rc2 = L->couple_group(set);
+      const int unroll = L->use_pot() ? L->pot_unroll() : 1;
+      for (int q = 0; q < unroll && rc2 == LCS_OK; q++) rc2 = L->couple_group(set);
+      // (counts the passes of this body)
       if (rc2 == LCS_OK)
         rc2 = L->launch("couple_continue", k_group_continue<T>, dim3(1), dim3(1), 0, L->grp_ptrs, (int)mem.size(),
-                        handle, L->max_loop_groups());
+                        handle, (L->max_loop_groups() + unroll - 1) / unroll);
       L->grp = nullptr;
       L->stream = s;
       if (rc2 != LCS_OK) rc2 = member_fail(L, rc2);

@@ -245,3 +245,32 @@ def test_halos_after_a_couple(dims, h, ov, precision):
         a = e.field_get(f, haloed=True)
         assert np.array_equal(a, np.pad(a[h:-h, h:-h, h:-h], h, mode="wrap")), f
     e.close()
+
+
+@pytest.mark.parametrize("precision", [F.PRECISION_FP64, F.PRECISION_FP32_MIXED])
+def test_group_members_leave_at_different_sweeps(precision, monkeypatch):
+    """The ensemble's loop (four groups a body from itrmax 24): members whose
+    couples end in different groups and bodies, after the first, second or third
+    sweep, each as alone, bit for bit."""
+    from lcs_b200 import _abi as abi
+
+    def configs(prec, n, count):
+        cfgs = plain(prec, n=n, count=count)
+        for c in cfgs:
+            c.itrmax, c.epsp = 70, 1e-3
+        return cfgs
+
+    def scaled(cfg, seed):
+        flow, parts = inputs(cfg, seed)
+        return [f * 0.25 * 3.0 ** (seed % 5) for f in flow], parts
+
+    plain, inputs = serve_cases.group_configs, serve_cases.inputs
+    monkeypatch.setattr(serve_cases, "group_configs", configs)
+    monkeypatch.setattr(serve_cases, "inputs", scaled)
+    sweeps = []
+    for i, c in enumerate(configs(precision, 28, 5)):
+        c.use_graphs = 1
+        logs = serve_cases.run_alone(Engine, c, 200 + i, 4)[2]
+        sweeps += [lg[k]["sweeps"] for lg in logs for k in ("couple1", "couple2")]
+    assert {s % 3 for s in sweeps} == {0, 1, 2} and max(sweeps) - min(sweeps) > 12 and min(sweeps) < 70, sweeps
+    serve_cases.check_group_equals_members_alone(Engine, abi.load_library(), precision, count=5, nsteps=2, n=28)
