@@ -404,10 +404,14 @@ LCS_API int lcs_step_poll(lcs_handle* h, int32_t* done);
 LCS_API int lcs_step_finish(lcs_handle* h, lcs_log* logs);
 /* Device bytes the handle holds (its pool), as lcs_footprint predicts. */
 LCS_API int lcs_device_bytes(lcs_handle* h, int64_t* bytes);
+/* How the handle's couples run (see lcs_flow_couple): 1 in potential form, 0
+ * as element-wise sweeps. */
+LCS_API int lcs_couple_form(lcs_handle* h, int32_t* form);
 /* Launch shapes of a handle, set from outside (no reference counterpart; the
  * batch's autotuner and the server use it): rw_rows = tile rows of the
- * HSMAC sweep (13, 8 or 5, or 29 in FP32: two rows a warp; 0 keeps the
- * current), zchunk = planes per z chunk
+ * element-wise HSMAC sweep (13, 8 or 5, or 29 in FP32: two rows a warp; 0 keeps
+ * the current; couples in potential form choose their tile by the grid and
+ * share, and no value changes them), zchunk = planes per z chunk
  * of a sweep (0: the built-in cost model), share = the part of the GPU the
  * handle's launches are sized for when several handles run at once (0, 1].
  * FP64 fields do not depend on these (the residual's partial sums are grouped
@@ -446,7 +450,8 @@ LCS_API int lcs_batch_member(lcs_batch* b, int32_t i, lcs_handle** h);
 LCS_API int lcs_batch_step(lcs_batch* b, int32_t nsteps, lcs_log* logs);
 /* The launch shapes lcs_batch_create chose for member i (see lcs_set_tuning):
  * its autotuner steps probe handles of each member shape together for every
- * candidate tile height and z chunk and keeps the fastest (probe_ms, one
+ * candidate tile height (element-wise sweeps; 0 where the couples run in
+ * potential form), z chunk and share and keeps the fastest (probe_ms, one
  * probe step); LCS_BATCH_TUNE=0 in the environment skips the probing. */
 LCS_API int lcs_batch_tuning(const lcs_batch* b, int32_t i, int32_t* rw_rows, int32_t* zchunk, double* share,
                              double* probe_ms);

@@ -283,6 +283,12 @@ int lcs_particles_density(lcs_handle* h, int32_t s, int32_t ratio, double* densi
   H(h);
   return h->e->particles_density(s, ratio, densities);
 }
+int lcs_couple_form(lcs_handle* h, int32_t* form) {
+  H(h);
+  if (!form) return LCS_EINVAL;
+  *form = h->e->couple_form();
+  return LCS_OK;
+}
 int lcs_set_tuning(lcs_handle* h, int32_t rw_rows, int32_t zchunk, double share) {
   H(h);
   return h->e->set_tuning(rw_rows, zchunk, share);

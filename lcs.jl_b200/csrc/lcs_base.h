@@ -52,6 +52,7 @@ struct EngineBase {
   virtual int step_poll(int* done) = 0;
   virtual int step_finish(lcs_log* logs) = 0;
   virtual int64_t device_bytes() const = 0;
+  virtual int couple_form() const = 0;
   virtual int set_tuning(int rw_rows, int zchunk, double share) = 0;
   virtual int flow_stat(lcs_flow_stats* out) = 0;
   virtual int particles_makeindex(int s, int stage, int grid_ratio) = 0;

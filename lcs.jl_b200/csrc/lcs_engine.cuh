@@ -1384,6 +1384,7 @@ class Engine : public EngineBase {
   // zchunk = planes per z chunk of the TMA sweeps (0: the cost model),
   // share = part of the GPU the launches are sized for (0 < share <= 1).
   // The step graphs are captured again with the new shapes.
+  int couple_form() const override { return use_pot() ? 1 : 0; }
   int set_tuning(int rw_rows, int zchunk, double share) override {
     if (async_pending) return fail(LCS_ESTATE, "asynchronous steps are in flight on this handle");
     if (rw_rows != 0 && rw_rows != 13 && rw_rows != 8 && rw_rows != 5 && rw_rows != 29)

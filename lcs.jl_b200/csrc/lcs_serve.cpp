@@ -83,10 +83,11 @@ bool probe_step(const std::vector<lcs_handle*>& probes, lcs_group* pg) {
 }
 
 // The batch's autotuner.  Members that share a shape (dims and precision) get
-// the same launch shapes: for every candidate (tile rows of the sweep x z
-// chunk x the part of the GPU a launch is sized for) it steps probe handles of
-// that shape, one per member, together (as one group when grouping is on;
-// zero fields, exactly 20 sweeps per couple, no particles) and times one
+// the same launch shapes: for every candidate (tile rows of the element-wise
+// sweep x z chunk x the part of the GPU a launch is sized for; couples in
+// potential form have no tile rows to choose) it steps probe handles of that
+// shape, one per member, together (as one group when grouping is on; zero
+// fields, a fixed number of sweeps per couple, no particles) and times one
 // step; the fastest candidate is applied to the members.  Probes never touch
 // a member's state, and no result depends on the launch shapes.
 int autotune(lcs_batch* b) {
@@ -118,7 +119,7 @@ int autotune(lcs_batch* b) {
     pc.mode = LCS_MODE_FLOW;
     pc.n_species = 0;
     pc.forcing = LCS_FORCING_NO;
-    pc.itrmin = pc.itrmax = 20;
+    pc.itrmin = pc.itrmax = ci.itrmax >= 24 ? 24 : 20;  // (from 24 on a couple's loop runs four groups a body)
     pc.use_graphs = 1;
     std::vector<lcs_handle*> probes;
     const int64_t n3 = (int64_t)ci.dims[0] * ci.dims[1] * ci.dims[2];
@@ -143,6 +144,8 @@ int autotune(lcs_batch* b) {
     // tile rows: FP32 also has 29-row tiles (two rows a warp)
     std::vector<int32_t> rows_c = {13, 8, 5};
     if (ci.precision == LCS_PRECISION_FP32_MIXED) rows_c.insert(rows_c.begin(), 29);
+    int32_t form = 0;
+    if (!probes.empty() && lcs_couple_form(probes[0], &form) == LCS_OK && form == 1) rows_c = {0};
     std::vector<int32_t> zc_c = {0};
     for (int d : {1, 2, 4})
       if (nz / d >= 8) zc_c.push_back((nz + 2) / d + 2);

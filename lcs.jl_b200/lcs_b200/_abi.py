@@ -271,6 +271,7 @@ PROTOTYPES = {
     "lcs_step_poll": (C.c_int, [_P, C.POINTER(C.c_int32)]),
     "lcs_step_finish": (C.c_int, [_P, C.POINTER(Log)]),
     "lcs_device_bytes": (C.c_int, [_P, _I64]),
+    "lcs_couple_form": (C.c_int, [_P, C.POINTER(C.c_int32)]),
     "lcs_set_tuning": (C.c_int, [_P, C.c_int32, C.c_int32, C.c_double]),
     "lcs_batch_create": (C.c_int, [C.POINTER(Config), C.c_int32, C.POINTER(_P)]),
     "lcs_batch_size": (C.c_int, [_P, C.POINTER(C.c_int32)]),

@@ -267,6 +267,12 @@ class Engine:
         self._check(self.lib.lcs_flow_couple(self.handle, stage, dtrk, C.byref(log)))
         return {"itr": log.itr, "sweeps": log.sweeps, "div": log.div}
 
+    def couple_form(self) -> str:
+        """How the handle's couples run: "potential" or "element-wise"."""
+        form = C.c_int32()
+        self._check(self.lib.lcs_couple_form(self.handle, C.byref(form)))
+        return "potential" if form.value else "element-wise"
+
     def forcing(self, dtrk: float) -> dict:
         """`Flows.forcing!` (src/flows/forcings)."""
         p = C.c_double()

@@ -1329,6 +1329,11 @@ int lcs_flow_stat(lcs_handle* h, lcs_flow_stats* o) {
 }
 
 /* Launch shapes do not exist on the CPU: checked and ignored. */
+int lcs_couple_form(lcs_handle* h, int32_t* form) {
+  if (!h || !form) return LCS_EINVAL;
+  *form = 0;
+  return LCS_OK;
+}
 int lcs_set_tuning(lcs_handle* h, int32_t rw_rows, int32_t zchunk, double share) {
   if (!h) return LCS_EINVAL;
   if ((rw_rows != 0 && rw_rows != 13 && rw_rows != 8 && rw_rows != 5) || zchunk < 0 || !(share > 0.0 && share <= 1.0))

@@ -56,3 +56,16 @@ def test_group_rejects_mixed_shapes():
     assert lib.lcs_group_create(hs, 2, C.byref(grp)) == _abi.EINVAL
     a.close()
     b.close()
+
+
+def test_batch_tuning_reports_what_was_chosen():
+    """Tile rows are a choice for element-wise couples only: members in
+    potential form report none, and their probes do not repeat equal launches."""
+    from helpers import make_config
+    from lcs_b200 import Batch
+
+    f32, f64 = _abi.PRECISION_FP32_MIXED, _abi.PRECISION_FP64
+    b = Batch([make_config(n, mode=_abi.MODE_FLOW, itrmax=30, precision=p) for n, p in ((24, f64), (24, f32), (48, f64))])
+    assert [e.couple_form() for e in b.members] == ["element-wise", "potential", "potential"]
+    assert [b.tuning(i)["rw_rows"] for i in range(3)][1:] == [0, 0] and b.tuning(0)["rw_rows"] in (13, 8, 5)
+    b.close()
