@@ -82,113 +82,133 @@ bool probe_step(const std::vector<lcs_handle*>& probes, lcs_group* pg) {
   return ok;
 }
 
-// The batch's autotuner.  Members that share a shape (dims and precision) get
-// the same launch shapes: for every candidate (tile rows of the element-wise
-// sweep x z chunk x the part of the GPU a launch is sized for; couples in
-// potential form have no tile rows to choose) it steps probe handles of that
-// shape, one per member, together (as one group when grouping is on; zero
-// fields, a fixed number of sweeps per couple, no particles) and times one
+// Members that share a shape (dims and precision): they get the same launch shapes.
+struct TuneShape {
+  std::vector<size_t> members;
+  double share = 1.0;  // of the ensemble's cells, one member's
+  MemberTuning best;
+};
+
+// Tries the candidates on probe handles of the shape and keeps the fastest in
+// t.best (its probe_ms stays 1e300 when no probe could run); `whole`: only the
+// one that sizes a launch for the whole GPU.
+void tune_shape(const lcs_batch* b, TuneShape& t, bool one_shape, bool whole) {
+  const lcs_config& ci = b->cfgs[t.members[0]];
+  lcs_config pc = ci;  // the probe: flow only, unforced (zero fields), a fixed sweep count
+  pc.mode = LCS_MODE_FLOW;
+  pc.n_species = 0;
+  pc.forcing = LCS_FORCING_NO;
+  pc.itrmin = pc.itrmax = ci.itrmax >= 24 ? 24 : 20;  // (from 24 on a couple's loop runs four groups a body)
+  pc.use_graphs = 1;
+  std::vector<lcs_handle*> probes;
+  const int64_t n3 = (int64_t)ci.dims[0] * ci.dims[1] * ci.dims[2];
+  std::vector<double> zero((size_t)n3, 0.0);
+  for (size_t q = 0; q < t.members.size(); q++) {
+    lcs_handle* h = nullptr;
+    if (lcs_create(&pc, &h) != LCS_OK) break;
+    if (lcs_upload_flow(h, zero.data(), zero.data(), zero.data(), zero.data()) != LCS_OK) {
+      lcs_destroy(h);
+      break;
+    }
+    probes.push_back(h);
+  }
+  lcs_group* pg = nullptr;
+  if (grouping_enabled() && probes.size() >= 2 && probes.size() <= 64 &&
+      lcs_group_create(probes.data(), (int32_t)probes.size(), &pg) != LCS_OK)
+    pg = nullptr;
+  const int nz = ci.dims[2];
+  // tile rows: FP32 also has 29-row tiles (two rows a warp)
+  std::vector<int32_t> rows_c = {13, 8, 5};
+  if (ci.precision == LCS_PRECISION_FP32_MIXED) rows_c.insert(rows_c.begin(), 29);
+  int32_t form = 0;
+  if (!probes.empty() && lcs_couple_form(probes[0], &form) == LCS_OK && form == 1) rows_c = {0};
+  std::vector<int32_t> zc_c = {0};
+  for (int d : {1, 2, 4})
+    if (nz / d >= 8) zc_c.push_back((nz + 2) / d + 2);
+  // candidates: tile rows x (the cost model sized for the member's share or
+  // for the whole GPU, or a fixed chunk)
+  struct Cand { int32_t rows, zc; double share; };
+  std::vector<Cand> cands;
+  // a grouped launch covers every member of the shape: each member's share of it
+  const double share_m = std::max(1e-3, t.share / (double)std::max<size_t>(1, t.members.size()));
+  for (int32_t rows : rows_c) {
+    if (!whole) cands.push_back({rows, 0, t.share});
+    if (one_shape || whole) cands.push_back({rows, 0, 1.0});
+    if (whole) continue;
+    if (pg) cands.push_back({rows, 0, share_m});
+    for (int32_t zc : zc_c)
+      if (zc > 0) cands.push_back({rows, zc, pg ? share_m : t.share});
+  }
+  for (const Cand& cd : cands) {
+    bool ok = !probes.empty();
+    for (lcs_handle* h : probes) ok = ok && lcs_set_tuning(h, cd.rows, cd.zc, cd.share) == LCS_OK;
+    for (int rep = 0; ok && rep < 2; rep++) {  // rep 0 captures the graphs; rep 1 is timed
+      const auto t0 = Clock::now();
+      ok = probe_step(probes, pg);
+      const double ms = std::chrono::duration<double, std::milli>(Clock::now() - t0).count();
+      if (ok && rep == 1 && ms < t.best.probe_ms) {
+        t.best.rw_rows = cd.rows;
+        t.best.zchunk = cd.zc;
+        t.best.share = cd.share;
+        t.best.probe_ms = ms;
+      }
+    }
+  }
+  if (pg) lcs_group_destroy(pg);
+  for (lcs_handle* h : probes) lcs_destroy(h);
+}
+
+// The batch's autotuner.  For every shape and every candidate (tile rows of the
+// element-wise sweep x z chunk x the part of the GPU a launch is sized for;
+// couples in potential form have no tile rows to choose) it steps probe handles
+// of that shape, one per member, together (as one group when grouping is on;
+// zero fields, a fixed number of sweeps per couple, no particles) and times one
 // step; the fastest candidate is applied to the members.  Probes never touch
 // a member's state, and no result depends on the launch shapes.
+//
+// Launches sized for the whole GPU are faster alone.  Beside other shapes they
+// cost the ensemble more than they give (12 FP32 members of 32^3 to 96^3: 32.8 ms
+// a step against 24.4; 12 FP64 ones of 16^3 to 32^3 6.6 and 6.1), except where a
+// single member sized for its part is the ensemble's longest chain and holds few
+// of its cells (96^3 and 32^3 in FP32: 11.0 ms and 12.9; 48^3, 64^3 and 96^3 in
+// FP64: 16.0 and 17.5; several members of the longest shape, 20^3 among the 12
+// above: 6.4 and 6.15): they are a candidate for one shape alone, and there.
 int autotune(lcs_batch* b) {
   const size_t m = b->members.size();
   double total_cells = 0.0;
   for (const auto& c : b->cfgs) total_cells += (double)c.dims[0] * c.dims[1] * c.dims[2];
-  std::vector<bool> done(m, false);
-  // With other shapes beside them a shape's launches are sized for its part of
-  // the GPU: sized for all of it each is faster alone, and the ensemble slower
-  // (12 members of 4 sizes: 32.5 ms a step against 23.5).
-  bool one_shape = true;
-  for (const auto& c : b->cfgs)
-    for (int a = 0; a < 3; a++) one_shape = one_shape && c.dims[a] == b->cfgs[0].dims[a] && c.precision == b->cfgs[0].precision;
+  std::vector<TuneShape> shapes;
   for (size_t i = 0; i < m; i++) {
-    if (done[i]) continue;
     const lcs_config& ci = b->cfgs[i];
-    std::vector<size_t> group;
-    for (size_t q = i; q < m; q++) {
-      const lcs_config& cq = b->cfgs[q];
+    TuneShape* at = nullptr;
+    for (auto& t : shapes) {
+      const lcs_config& cq = b->cfgs[t.members[0]];
       if (cq.dims[0] == ci.dims[0] && cq.dims[1] == ci.dims[1] && cq.dims[2] == ci.dims[2] &&
-          cq.precision == ci.precision) {
-        group.push_back(q);
-        done[q] = true;
-      }
+          cq.precision == ci.precision)
+        at = &t;
     }
-    const double cells = (double)ci.dims[0] * ci.dims[1] * ci.dims[2];
-    const double share = std::min(1.0, std::max(1e-3, cells / total_cells));
-    lcs_config pc = ci;  // the probe: flow only, unforced (zero fields), a fixed sweep count
-    pc.mode = LCS_MODE_FLOW;
-    pc.n_species = 0;
-    pc.forcing = LCS_FORCING_NO;
-    pc.itrmin = pc.itrmax = ci.itrmax >= 24 ? 24 : 20;  // (from 24 on a couple's loop runs four groups a body)
-    pc.use_graphs = 1;
-    std::vector<lcs_handle*> probes;
-    const int64_t n3 = (int64_t)ci.dims[0] * ci.dims[1] * ci.dims[2];
-    std::vector<double> zero((size_t)n3, 0.0);
-    for (size_t q = 0; q < group.size(); q++) {
-      lcs_handle* h = nullptr;
-      if (lcs_create(&pc, &h) != LCS_OK) break;
-      if (lcs_upload_flow(h, zero.data(), zero.data(), zero.data(), zero.data()) != LCS_OK) {
-        lcs_destroy(h);
-        break;
-      }
-      probes.push_back(h);
+    if (!at) {
+      shapes.emplace_back();
+      at = &shapes.back();
+      at->share = std::min(1.0, std::max(1e-3, (double)ci.dims[0] * ci.dims[1] * ci.dims[2] / total_cells));
+      at->best.share = at->share;
+      at->best.probe_ms = 1e300;
     }
-    lcs_group* pg = nullptr;
-    if (grouping_enabled() && probes.size() >= 2 && probes.size() <= 64 &&
-        lcs_group_create(probes.data(), (int32_t)probes.size(), &pg) != LCS_OK)
-      pg = nullptr;
-    MemberTuning best;
-    best.share = share;
-    best.probe_ms = 1e300;
-    const int nz = ci.dims[2];
-    // tile rows: FP32 also has 29-row tiles (two rows a warp)
-    std::vector<int32_t> rows_c = {13, 8, 5};
-    if (ci.precision == LCS_PRECISION_FP32_MIXED) rows_c.insert(rows_c.begin(), 29);
-    int32_t form = 0;
-    if (!probes.empty() && lcs_couple_form(probes[0], &form) == LCS_OK && form == 1) rows_c = {0};
-    std::vector<int32_t> zc_c = {0};
-    for (int d : {1, 2, 4})
-      if (nz / d >= 8) zc_c.push_back((nz + 2) / d + 2);
-    // candidates: tile rows x (the cost model sized for the member's share or
-    // for the whole GPU, or a fixed chunk)
-    struct Cand { int32_t rows, zc; double share; };
-    std::vector<Cand> cands;
-    // a grouped launch covers every member of the shape: each member's share of it
-    const double share_m = std::max(1e-3, share / (double)std::max<size_t>(1, group.size()));
-    for (int32_t rows : rows_c) {
-      cands.push_back({rows, 0, share});
-      if (one_shape) cands.push_back({rows, 0, 1.0});
-      if (pg) cands.push_back({rows, 0, share_m});
-      for (int32_t zc : zc_c)
-        if (zc > 0) cands.push_back({rows, zc, pg ? share_m : share});
-    }
-    for (const Cand& cd : cands) {
-      bool ok = !probes.empty();
-      for (lcs_handle* h : probes) ok = ok && lcs_set_tuning(h, cd.rows, cd.zc, cd.share) == LCS_OK;
-      for (int rep = 0; ok && rep < 2; rep++) {  // rep 0 captures the graphs; rep 1 is timed
-        const auto t0 = Clock::now();
-        ok = probe_step(probes, pg);
-        const double ms = std::chrono::duration<double, std::milli>(Clock::now() - t0).count();
-        if (ok && rep == 1 && ms < best.probe_ms) {
-          best.rw_rows = cd.rows;
-          best.zchunk = cd.zc;
-          best.share = cd.share;
-          best.probe_ms = ms;
-        }
-      }
-    }
-    if (pg) lcs_group_destroy(pg);
-    for (lcs_handle* h : probes) lcs_destroy(h);
-    if (best.probe_ms >= 1e300) {  // no probe could run: the built-in shapes
-      best.rw_rows = 0;
-      best.zchunk = 0;
-      best.share = 1.0;
-      best.probe_ms = 0.0;
-    }
-    for (size_t q : group) {
-      const int rc = lcs_set_tuning(b->members[q], best.rw_rows, best.zchunk, best.share);
+    at->members.push_back(i);
+  }
+  TuneShape* longest = &shapes[0];
+  for (auto& t : shapes) {
+    tune_shape(b, t, shapes.size() == 1, false);
+    if (t.best.probe_ms > longest->best.probe_ms) longest = &t;
+  }
+  if (shapes.size() > 1 && longest->best.probe_ms < 1e300 && longest->members.size() == 1 && longest->share < 0.5)
+    tune_shape(b, *longest, false, true);
+  for (auto& t : shapes) {
+    if (t.best.probe_ms >= 1e300) t.best = MemberTuning();  // no probe could run: the built-in shapes
+    for (size_t q : t.members) {
+      const int rc = lcs_set_tuning(b->members[q], t.best.rw_rows, t.best.zchunk, t.best.share);
       if (rc != LCS_OK) return serve_fail(rc, "batch member " + std::to_string(q) + ": " + handle_error(b->members[q]));
-      b->tuning[q] = best;
+      b->tuning[q] = t.best;
     }
   }
   return LCS_OK;
