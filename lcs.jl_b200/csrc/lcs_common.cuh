@@ -118,6 +118,13 @@ struct Ctx {
   int pot_age, pot_check;
 };
 
+// HSMAC coefficients (src/flows/couples/hsmac.jl)
+struct HsmacCoef {
+  double dxi, dyi, dzi, dl, omega, dxmin, epsp, count;  // count = (n+1)^3
+  int itrmin, itrmax;
+  int coloring;  // enum lcs_coloring
+};
+
 // ---- stencil primitives (src/diff.jl:1-39), same evaluation order --------
 template <typename T> __device__ __forceinline__ T interp_o2_at_half(T a, T b) { return T(0.5) * (a + b); }
 template <typename T> __device__ __forceinline__ T interp_o4_at_half(T a, T b, T c, T d) {

@@ -26,7 +26,7 @@
 #include "lcs_kernels.cuh"
 #include "lcs_tma.cuh"
 #include "lcs_hsmac_rw.cuh"
-#include "lcs_potential.cuh"
+#include "lcs_potential.h"
 #include "lcs_makeindex.cuh"
 #include "lcs_pstat.cuh"
 
@@ -336,11 +336,11 @@ class Engine : public EngineBase {
   // (FP64: 20 and 4): FP32 32^3 33, 27, 21; 48^3 33, 27, 24; 64^3 35, 31, 35;
   // 96^3 43, 37, 64; 128^3 60, 56, 122; 192^3 117, 127, 273; 256^3 240, 228;
   // 512^3 1044, 1199.  FP64 48^3 33, 29; 64^3 40, 41; 96^3 52, 77.
-  static constexpr int kPotW = sizeof(T) == 8 ? 8 : 12, kPotWS = sizeof(T) == 8 ? 8 : 16, kPotRS = sizeof(T) == 8 ? 4 : 2;
-  using PotT = PotTile<T, kPotW, 4>;        // FP64 20 output rows, FP32 36
-  using PotS = PotTile<T, kPotWS, kPotRS>;  // FP32 20 output rows (FP64: the same as PotT)
-  using PotV = PotTile<T, 8, 2>;            // 4 output rows
-  static constexpr size_t kSlabSmem = (size_t)10 * 1024 * sizeof(T);
+  using PotT = typename PotTiles<T>::Tall;
+  using PotS = typename PotTiles<T>::Mid;
+  using PotV = typename PotTiles<T>::Flat;
+  static constexpr size_t kSlabSmem = kPotSlabPlanes * 1024 * sizeof(T);
+  const PotKernels<T>& pot = pot_kernels(T());
   int init_pot() {
     const char* sweep = std::getenv("LCS_B200_FUSED_SWEEP");
     const std::string sw = sweep ? std::string(sweep) : std::string();
@@ -353,10 +353,10 @@ class Engine : public EngineBase {
              (size_t)ps.total * sizeof(T) <= (size_t)plan.stage_elems * sizeof(double) &&
              (sw == "potential" || (sw.empty() && !shaped && (sizeof(T) == 4 || cells > 40 * 40 * 40)));
     if (!pot_ok) return LCS_OK;
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotW, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotT::bytes));
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, kPotWS, kPotRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotS::bytes));
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_sweep<T, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PotV::bytes));
-    LCS_CUDA(cudaFuncSetAttribute(k_pot_slab<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
+    const size_t smem[3] = {PotT::bytes, PotS::bytes, PotV::bytes};
+    for (int q = 0; q < 3; q++)
+      LCS_CUDA(cudaFuncSetAttribute(pot.sweep[q], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[q]));
+    LCS_CUDA(cudaFuncSetAttribute(pot.slab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem));
     if (const char* t = std::getenv("LCS_B200_POT_TILE")) pot_tile = std::max(0, std::min(2, std::atoi(t)));
     pot_ptrs.ctx[0] = dctx;
     pot_ptrs.P[0] = P;
@@ -419,12 +419,12 @@ class Engine : public EngineBase {
   int pot_setup(int set) {
     const PotGeom pg = pot_geom();
     const int64_t half = (int64_t)g.n[0] / 2 * g.n[1] * g.n[2];
-    return launch("pot_setup", k_pot_setup<T>, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
+    return launch("pot_setup", pot.setup, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
   }
   int pot_apply(int set) {
     const PotGeom pg = pot_geom();
     const int64_t half = (int64_t)g.n[0] / 2 * g.n[1] * g.n[2];
-    return launch("pot_apply", k_pot_apply<T>, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
+    return launch("pot_apply", pot.apply, dim3(blocks_for(half, 256), pot_members()), dim3(256), 0, pot_args(), g, set, pg);
   }
   // FP32: the rounding of the stored velocity into the logged residual
   int pot_round(int set) {
@@ -432,7 +432,7 @@ class Engine : public EngineBase {
       return LCS_OK;
     } else {
       const dim3 grid(blocks_for((int64_t)g.n[0] * g.n[1] * g.n[2], 256), pot_members());
-      return launch("pot_round", k_pot_round<T>, grid, dim3(256), 0, pot_args(), g, set, pot_geom(), hc);
+      return launch("pot_round", pot.round, grid, dim3(256), 0, pot_args(), g, set, pot_geom(), hc);
     }
   }
   // one group of three sweeps
@@ -443,15 +443,13 @@ class Engine : public EngineBase {
     const int64_t faces = (int64_t)g.n[0] * g.n[1] + (int64_t)g.n[0] * g.n[2] + (int64_t)g.n[1] * g.n[2];
     // (FP32: it has all cells to visit when it measures the velocity's rounding)
     const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2], jump = sizeof(T) == 4 ? std::max(faces, cells / 4) : faces;
-    LCS_TRY(launch("pot_jump", k_pot_jump<T>, dim3(blocks_for(jump, 256), M), dim3(256), 0, pot_args(), g, set, pg, hc));
+    LCS_TRY(launch("pot_jump", pot.jump, dim3(blocks_for(jump, 256), M), dim3(256), 0, pot_args(), g, set, pg, hc));
     if (cfg.overlap)
-      LCS_TRY(launch("pot_slab", k_pot_slab<T>, dim3(pg.nslab, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg));
+      LCS_TRY(launch("pot_slab", pot.slab, dim3(pg.nslab, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg));
     const dim3 grid(pg.nseg, M);
-    if (pg.kind == 2)
-      return launch("pot_sweep", k_pot_sweep<T, 8, 2>, grid, dim3(PotV::NT), PotV::bytes, pot_args(), pg, hc, loop);
-    if (pg.kind == 1)
-      return launch("pot_sweep", k_pot_sweep<T, kPotWS, kPotRS>, grid, dim3(PotS::NT), PotS::bytes, pot_args(), pg, hc, loop);
-    return launch("pot_sweep", k_pot_sweep<T, kPotW, 4>, grid, dim3(PotT::NT), PotT::bytes, pot_args(), pg, hc, loop);
+    const dim3 block(pg.kind == 0 ? PotT::NT : pg.kind == 1 ? PotS::NT : PotV::NT);
+    const size_t smem = pg.kind == 0 ? PotT::bytes : pg.kind == 1 ? PotS::bytes : PotV::bytes;
+    return launch("pot_sweep", pot.sweep[pg.kind], grid, block, smem, pot_args(), pg, hc, loop);
   }
 
   // ---------------------------------------------------------- tensor maps

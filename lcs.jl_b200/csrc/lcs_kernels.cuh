@@ -269,12 +269,6 @@ __global__ void k_update(const Ctx* __restrict__ ctx, Grid g, int out_set, int u
 // --------------------------------------------------------------------------
 // HSMAC (src/flows/couples/hsmac.jl)
 // --------------------------------------------------------------------------
-struct HsmacCoef {
-  double dxi, dyi, dzi, dl, omega, dxmin, epsp, count;  // count = (n+1)^3
-  int itrmin, itrmax;
-  int coloring;  // enum lcs_coloring
-};
-
 // Colour of a cell in the swept box, or -1 when the colouring never visits
 // it: RedBlackFast visits every cell with (i+j+k) mod 2 == colour
 // (lib/parallel/src/foraxes.jl:93-107); RedBlack tests `sum(i) % 2 == colour`

@@ -30,7 +30,10 @@
 // beforehand, in place, from the core cells next to them, which it computes too.
 #pragma once
 
+#include "../../include/lcs_b200.h"
+#include "lcs_kernels.cuh"
 #include "lcs_hsmac_rw.cuh"
+#include "lcs_potential.h"
 
 namespace lcs {
 namespace {
@@ -52,72 +55,6 @@ template <typename T>
 __device__ __forceinline__ T pot_div(T x, T sx, T sy, T sz, T d, T cx, T cy, T cz) {
   return pfma<T>(cx, pfma<T>(T(2), x, -sx), pfma<T>(cy, pfma<T>(T(2), x, -sy), pfma<T>(cz, pfma<T>(T(2), x, -sz), d)));
 }
-
-constexpr int kPotLayers = 7;  // layers next to a face kept compact: n-2, n-1, n, 1, 2, 3, 4
-constexpr int kPotDLayers = 5; // of D along x: n-1, n, 1, 2, 3
-constexpr int kPotSlab = 22;   // a slab tile's own columns (32 less 5 on each side)
-constexpr int kPotSlabThreads = 1024;
-
-// Layout of Phi and D (each in one of the spare velocity buffers): positions
-// -1 .. n+3 along each axis, x fastest, rows on 32-byte boundaries; an odd x
-// starts an aligned pair.  Offsets (elements of T) of the couple's small
-// arrays in its scratch.
-struct PotScratch {
-  int nx, ny, nz, px;   // px: row pitch
-  int pz;               // plane pitch (a field holds < 2^31 elements)
-  int64_t l[3], dx, e[3], j[3], total;
-  __host__ __device__ __forceinline__ int at(int i, int j, int k) const { return (k + 1) * pz + (j + 1) * px + (i + 1); }
-};
-__host__ __device__ inline PotScratch pot_scratch(const int n[3], int elem) {
-  PotScratch p;
-  p.nx = n[0];
-  p.ny = n[1];
-  p.nz = n[2];
-  const int a = 32 / elem;
-  p.px = (n[0] + 6 + a - 1) / a * a;
-  p.pz = p.px * (n[1] + 5);
-  const int64_t x = n[0], y = n[1], z = n[2];
-  const int64_t face[3] = {y * z, x * z, x * y};
-  int64_t o = 0;
-  for (int a3 = 0; a3 < 3; a3++) {  // Phi next to the faces: [7][nz][ny], [7][nz][nx], [7][ny][nx]
-    p.l[a3] = o;
-    o += kPotLayers * face[a3];
-  }
-  p.dx = o;  // [5][nz][ny]
-  o += kPotDLayers * face[0];
-  for (int a3 = 0; a3 < 3; a3++) {  // Phi of the cells n+1 after a group: [nz][ny], [nz][nx], [ny][nx]
-    p.e[a3] = o;
-    o += face[a3];
-  }
-  for (int a3 = 0; a3 < 3; a3++) {  // the jumps, same shapes
-    p.j[a3] = o;
-    o += face[a3];
-  }
-  p.total = o;
-  return p;
-}
-
-// Handles that run the same launches side by side (one for a run alone).
-constexpr int kPotMax = 64;
-template <typename T>
-struct PotGroup {
-  Ctx* ctx[kPotMax];
-  T* P[kPotMax];
-  T* scratch[kPotMax];
-  double* partials[kPotMax];
-};
-
-struct PotGeom {
-  PotScratch s;
-  int overlap;
-  int kind, gx, gy;        // tile of k_pot_sweep (host's choice), tile columns along x and y
-  int nseg, nc;            // CTAs; z chunks of a column
-  int slab_part, nslab;    // residual partials of the slab tiles: first, count
-  int slab0[3];            // first tile of an axis's slabs (z, y, x in turn)
-  double cx, cy, cz, wd;     // 1/dx^2 .., -omega dl
-  double dxi, dyi, dzi;
-  double exit_sum;         // the exit test's bound on a sweep's sum of div^2 (a hair above it)
-};
 
 __device__ __forceinline__ int pot_wrap(int i, int n) {  // 1-based image of i in -n < i
   i = i < 1 ? i + n : i;
@@ -555,45 +492,24 @@ __device__ __forceinline__ void pot_slab_body(const PotGroup<T>& ga, const PotGe
 // blocks: the tiles of the z slabs, then of the y and x slabs (slab0: first tile of each axis)
 template <typename T>
 __global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_constant__ PotGroup<T> ga, PotGeom pg) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char pot_smem[];
   __shared__ double red[32];
   const int m = blockIdx.y, b = blockIdx.x;
   const Ctx* ctx = ga.ctx[m];
   // (a group that runs again finds these in place)
   const int done = ctx->cs.done, cont = ctx->cs.cont, redo = ctx->pot_redo, check = ctx->pot_check;
   if (done || !cont || redo || check) return;
-  T* sh = (T*)smem_raw;  // [10][32][32]
+  T* sh = (T*)pot_smem;  // [10][32][32]
   if (b < pg.slab0[1]) pot_slab_body<T, 2>(ga, pg, m, b, sh, red);
   else if (b < pg.slab0[0]) pot_slab_body<T, 1>(ga, pg, m, b - pg.slab0[1], sh, red);
   else pot_slab_body<T, 0>(ga, pg, m, b - pg.slab0[0], sh, red);
 }
-
-constexpr int kPotMaxChunk = 1024, kPotMaxPlanes = kPotMaxChunk + 24;
 
 // Zero where a mask word is zero (a select without a branch, also for NaN).
 __device__ __forceinline__ float pot_keep(float v, int mask) { return __int_as_float(__float_as_int(v) & mask); }
 __device__ __forceinline__ double pot_keep(double v, int mask) {
   return __hiloint2double(__double2hiint(v) & mask, __double2loint(v) & mask);
 }
-
-// Tile of k_pot_sweep: NW warps of RW rows (RW even); a lane owns an x-pair.
-template <typename T, int NW, int RW>
-struct PotTile {
-  static constexpr int NT = 32 * NW, ROWS = NW * RW;
-  static constexpr int TX = 52, TY = ROWS - 12;  // outputs: 6 cells less on every side
-  static constexpr size_t d_elems = (size_t)6 * 2 * ROWS * 32;   // D of 6 planes, split by colour
-  static constexpr size_t x_elems = (size_t)2 * 6 * NW * 2 * 32; // rows at the warps' edges, double buffered
-  static constexpr size_t bytes = (d_elems + x_elems) * sizeof(T) + kPotMaxPlanes * sizeof(int);
-  static_assert(RW % 2 == 0, "a warp's first row has the same parity in every warp");
-};
-
-// The loop of a couple inside a step graph: the last CTA of a group's sweep
-// sets its condition (a run alone; a batch group has a kernel for it, which
-// looks at all its members).
-struct PotLoop {
-  int on, max_groups;
-  cudaGraphConditionalHandle handle;
-};
 
 // Three red-black sweeps (six half sweeps) in one pass.
 //
@@ -630,12 +546,12 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   using T2 = pair_t<T>;
   constexpr int UF = 2;  // planes between two moves of the registers
   constexpr int NP = UF + 7;  // registers of a colour: planes t .. t - 7 and UF - 1 more
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char pot_smem[];
   __shared__ double red[32];
   __shared__ int last_flag;
-  T* sD = (T*)smem_raw;                // [6][2][ROWS][32]
-  T* sX = (T*)smem_raw + L::d_elems;   // [2][6][NW][2][32]
-  int* sZ = (int*)((T*)smem_raw + L::d_elems + L::x_elems);  // box bits of the planes kb - 13 ..
+  T* sD = (T*)pot_smem;                // [6][2][ROWS][32]
+  T* sX = (T*)pot_smem + L::d_elems;   // [2][6][NW][2][32]
+  int* sZ = (int*)((T*)pot_smem + L::d_elems + L::x_elems);  // box bits of the planes kb - 13 ..
   const int m = blockIdx.y;
   Ctx* ctx = ga.ctx[m];
   const int done = ctx->cs.done, cont = ctx->cs.cont, cur = ctx->pot_cur, redo = ctx->pot_redo, check = ctx->pot_check;
@@ -1003,6 +919,22 @@ __global__ void __launch_bounds__(256) k_pot_apply(const __grid_constant__ PotGr
             }
           }
   }
+}
+
+template <typename T>
+PotKernels<T> make_pot_kernels() {
+  using L = PotTiles<T>;
+  PotKernels<T> k;
+  k.setup = k_pot_setup<T>;
+  k.jump = k_pot_jump<T>;
+  k.slab = k_pot_slab<T>;
+  k.sweep[0] = k_pot_sweep<T, L::Tall::NW, L::Tall::RW>;
+  k.sweep[1] = k_pot_sweep<T, L::Mid::NW, L::Mid::RW>;
+  k.sweep[2] = k_pot_sweep<T, L::Flat::NW, L::Flat::RW>;
+  k.round = nullptr;
+  if constexpr (sizeof(T) == 4) k.round = k_pot_round<T>;
+  k.apply = k_pot_apply<T>;
+  return k;
 }
 
 }  // namespace
