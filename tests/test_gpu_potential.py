@@ -14,8 +14,9 @@ import numpy as np
 import pytest
 
 import serve_cases
+import test_gpu_parity as parity
 from helpers import make_config, rel_l2
-from lcs_b200 import Engine, _abi
+from lcs_b200 import Engine, LCSError, _abi
 from oracle_engine import OracleEngine
 
 F = _abi
@@ -41,9 +42,12 @@ def couple(cls, dims, ov, itrmin, itrmax, epsp, precision=F.PRECISION_FP64, stag
     return lg, out
 
 
-# the tiles give 52 x 20 columns and the slab tiles 26 x 26: one column or row
-# less, equal and more; few planes; the smallest grid; several tiles and chunks
-DIMS = [(8, 8, 8), (24, 26, 30), (50, 18, 40), (52, 20, 32), (54, 22, 20), (106, 42, 16), (72, 64, 130), (96, 96, 96)]
+# the sweep's tiles give 52 x 20 columns, of n + 1 (dims are even): just below,
+# and above one and two of them; few planes; the smallest grid; several tiles and
+# chunks.  A slab tile gives 22 x 22 of n + 5 or n - 1: 22 | 24 and 44 | 46 (n - 1),
+# 38 | 40 (n + 5) lie on either side, along each axis.
+DIMS = [(8, 8, 8), (24, 26, 30), (50, 18, 40), (52, 20, 32), (54, 22, 20), (106, 42, 16), (72, 64, 130), (96, 96, 96),
+        (22, 38, 44), (24, 40, 46), (44, 22, 38), (46, 24, 40), (38, 44, 22), (40, 46, 24)]
 
 
 @pytest.mark.parametrize("ov", [True, False])
@@ -274,3 +278,60 @@ def test_group_members_leave_at_different_sweeps(precision, monkeypatch):
         sweeps += [lg[k]["sweeps"] for lg in logs for k in ("couple1", "couple2")]
     assert {s % 3 for s in sweeps} == {0, 1, 2} and max(sweeps) - min(sweeps) > 12 and min(sweeps) < 70, sweeps
     serve_cases.check_group_equals_members_alone(Engine, abi.load_library(), precision, count=5, nsteps=2, n=28)
+
+
+@pytest.mark.parametrize("tile", ["0", "2"])
+@pytest.mark.parametrize("ov", [True, False])
+def test_fp64_planes_without_masks(ov, tile, monkeypatch):
+    """Interior tiles of one long z chunk: most planes run the form without
+    masks (three tile columns, so that the middle one lies off both faces)."""
+    monkeypatch.setenv("LCS_B200_POT_TILE", tile)
+    monkeypatch.setenv("LCS_B200_ZCHUNK", "60")
+    dims = (160, 64, 48)
+    lg, g = couple(Engine, dims, ov, 6, 13, 1e-12)
+    lo, o = couple(OracleEngine, dims, ov, 6, 13, 1e-12)
+    assert lg["sweeps"] == lo["sweeps"] and abs(lg["div"] - lo["div"]) <= 1e-9 * lo["div"]
+    for a, b in zip(g, o):
+        assert rel_l2(a, b) <= 1e-12
+
+
+@pytest.mark.parametrize("graphs", [0, 1])
+def test_ten_steps_noncubic(graphs):
+    """Whole steps (forcing, particles) of FP64 boxes that run element by element
+    unless asked: the bounds of the element-wise form, 1e-10 after ten steps."""
+    parity.test_ten_steps_noncubic_rel_l2(graphs)
+
+
+@pytest.mark.parametrize("forcing", [F.FORCING_LINEAR_POWER, F.FORCING_RC_ENERGY, F.FORCING_NO])
+@pytest.mark.parametrize("ov", [True, False])
+def test_ten_steps(forcing, ov):
+    cfg = make_config(32, forcing=forcing, power=0.5, energy=0.649, kmin=1, kmax=2, coarse=8, Re=100.0, overlap=ov,
+                      itrmin=6, itrmax=40, epsp=1e-8 * 2 * np.pi / 32, graphs=1,
+                      species=[{"n": 2000, "density_ratio": 843.0}, {"n": 1000, "density_ratio": 843.0}])
+    (g, o), (lg, lo) = parity.evolve_pair(cfg, 10, nparts=(2000, 1000), graphs=True)
+    assert g.couple_form() == "potential"
+    for a, b in zip(lg, lo):
+        assert [a[c]["itr"] for c in ("couple1", "couple2")] == [b[c]["itr"] for c in ("couple1", "couple2")]
+        assert abs(a["dt"] - b["dt"]) <= 1e-13 * b["dt"]
+    for a, b in zip(g.download_flow(), o.download_flow()):
+        assert rel_l2(a, b) <= 1e-10
+    for q in (0, 1):
+        a, b = g.download_particles(q), o.download_particles(q)
+        assert all(rel_l2(a[k], b[k]) <= 1e-10 for k in ("x", "y", "z", "u", "v", "w"))
+
+
+@pytest.mark.parametrize("graphs", [0, 1])
+@pytest.mark.parametrize("precision", [F.PRECISION_FP64, F.PRECISION_FP32_MIXED])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_nonfinite_residual_is_reported(bad, precision, graphs):
+    """A non-finite P leaves the time step finite and reaches the couple through
+    the rhs: the loop ends and the call reports it."""
+    e = Engine(make_config(24, mode=F.MODE_FLOW, Re=50.0, itrmin=6, itrmax=60, graphs=graphs, precision=precision))
+    rng = np.random.default_rng(1)
+    flow = [rng.standard_normal(e.interior_shape) * 0.3 for _ in range(4)]
+    flow[3][5, 6, 7] = bad
+    e.upload_flow(*flow)
+    with pytest.raises(LCSError) as ei:
+        e.step(1)
+    assert ei.value.code == F.ENONFINITE
+    e.close()

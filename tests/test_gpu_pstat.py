@@ -156,3 +156,22 @@ def test_rdf_reach(tol, radius, cells):
         e.close()
     a, b = out
     assert np.array_equal(a["npairs"], b["npairs"]) and a["npairs_contact"] == b["npairs_contact"]
+
+
+@pytest.mark.parametrize("cells", [1, 2])
+def test_rdf_particles_in_the_outer_cells(cells):
+    """Positions a little outside the box lie in the cells 0 and nc + 1 of the
+    axes 0:nc+1 and count as neighbours: no cell is left out for its distance."""
+    cfg = make_config(32, species=[{"n": 3000, "density_ratio": 843.0}], Re=50.0)
+    out = []
+    for cls in (Engine, OracleEngine):
+        e = cls(cfg)
+        rng = np.random.default_rng(9)
+        x, y, z = (rng.random(3000) * (L + 0.6) - 0.3 for _ in range(3))  # a cell is 0.785 wide
+        zero = np.zeros(3000)
+        e.upload_particles(0, np.full(3000, 0.125), x, y, z, zero, zero, zero, ids=np.arange(1, 3001))
+        out.append(e.particles_stat(0, 1.0, search_cell_size=cells, contact_tolerance=0.5, min_radius=1e-3,
+                                    max_wavenumber=1, nsamples=2)["rdf"])
+        e.close()
+    a, b = out
+    assert np.array_equal(a["npairs"], b["npairs"]) and a["npairs_contact"] == b["npairs_contact"] > 0
