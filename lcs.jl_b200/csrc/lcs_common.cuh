@@ -71,7 +71,7 @@ struct CoupleState {
   int itr;      // reference `itr`
   int sweeps;   // sweeps executed
   int done;     // exit criterion met
-  int cont;     // WHILE-loop condition value (itr < itrmax && !done)
+  int cont;     // WHILE-loop condition value (itr < itrmax && !done); 2: the group at hand is passed over (k_pot_jump)
   int groups;   // iterations of the graph's WHILE loop so far (bounds it)
   double div;   // last residual
   double sum;   // last sum of div^2
@@ -110,12 +110,11 @@ struct Ctx {
   int pot_pending;  // the last group's jumps are not yet in the right-hand side
   int pot_redo;     // sweeps of the group to run again (the exit lay inside it), 0: none
   // FP32 only, see k_pot_jump: what the residual's sum has to have added for the
-  // rounding of the stored velocity (0: not measured in this couple),
-  // groups since it was measured, residual sums of the last group, and the
-  // state of exit tests that wait for it (1: to be measured, 2: tested, the
-  // rest of this group does nothing).
+  // rounding of the stored velocity (0: not measured in this couple), itr when
+  // it was measured, the last group's residual sums, and whether its exit tests
+  // wait for the measurement.
   double pot_round, pot_sum[3];
-  int pot_age, pot_check;
+  int pot_since, pot_check;
 };
 
 // HSMAC coefficients (src/flows/couples/hsmac.jl)

@@ -431,7 +431,7 @@ class Engine : public EngineBase {
     if constexpr (sizeof(T) == 8) {
       return LCS_OK;
     } else {
-      const dim3 grid(blocks_for((int64_t)g.n[0] * g.n[1] * g.n[2], 256), pot_members());
+      const dim3 grid(blocks_for((int64_t)g.n[0] / 2 * g.n[1] * g.n[2], 256), pot_members());
       return launch("pot_round", pot.round, grid, dim3(256), 0, pot_args(), g, set, pot_geom(), hc);
     }
   }
@@ -443,7 +443,8 @@ class Engine : public EngineBase {
     const int64_t faces = (int64_t)g.n[0] * g.n[1] + (int64_t)g.n[0] * g.n[2] + (int64_t)g.n[1] * g.n[2];
     // (FP32: it has all cells to visit when it measures the velocity's rounding)
     const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2], jump = sizeof(T) == 4 ? std::max(faces, cells / 4) : faces;
-    LCS_TRY(launch("pot_jump", pot.jump, dim3(blocks_for(jump, 256), M), dim3(256), 0, pot_args(), g, set, pg, hc));
+    LCS_TRY(launch("pot_jump", pot.jump, dim3(blocks_for(jump, 256), M), dim3(256), 0, pot_args(), g, set, pg, hc,
+                   loop));
     if (cfg.overlap)
       LCS_TRY(launch("pot_slab", pot.slab, dim3(pg.nslab, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg));
     const dim3 grid(pg.nseg, M);

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) k_pot_setup(const __grid_constant__ PotGr
     ctx->pot_pending = 0;
     ctx->pot_redo = 0;
     ctx->pot_round = 0.0;
-    ctx->pot_age = 0;
+    ctx->pot_since = 0;
     ctx->pot_check = 0;
   }
 }
@@ -146,7 +146,7 @@ __device__ __forceinline__ void pot_exit(Ctx* ctx, const HsmacCoef& cf, const do
 // divergence of the velocity as it would be stored for the potential `phi` (a
 // group's output, its jumps pending) less the divergence that the sweeps see
 // there.  It holds every rounding between the two: of the velocity's faces, of
-// D and of the sweeps' own sums.  Bound by the latency of its 14 loads a cell.
+// D and of the sweeps' own sums.  Bound by the latency of its loads.
 template <typename T>
 __device__ __forceinline__ double pot_round_sum(const Ctx* ctx, const Grid& g, int set, const T* __restrict__ phi,
                                                 const T* __restrict__ s, const PotGeom& pg) {
@@ -157,57 +157,62 @@ __device__ __forceinline__ double pot_round_sum(const Ctx* ctx, const Grid& g, i
   const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz, px = pg.s.px, pz = pg.s.pz;
   const T cx = (T)pg.cx, cy = (T)pg.cy, cz = (T)pg.cz;
   double acc = 0.0;
-  const int total = nx * ny * nz;  // < 2^31 (host)
-  for (int64_t t64 = (int64_t)blockIdx.x * 256 + threadIdx.x; t64 < total; t64 += (int64_t)gridDim.x * 256) {
-    const int t = (int)t64;
-    const int i = 1 + t % nx, r = t / nx, j = 1 + r % ny, k = 1 + r / ny;
+  const int hx = nx / 2, total = hx * ny * nz;  // < 2^31 (host)
+  // of a cell and an axis: the divergence of its two faces as stored, and the
+  // sum of its two neighbours as the sweeps see them.  lo, hi: the neighbours'
+  // images; a, b: the low and the high face's velocity; first, last: the cell
+  // lies there, f: its place on that face.
+  auto axis = [&](int ax, T p, T lo, T hi, T a, T b, bool first, bool last, int f, double di, T* nsum) {
+    T vlo = p, vhi = hi;  // the high neighbour of the low face's cell, and of this one, as k_pot_apply has them
+    T slo = lo, shi = hi;
+    if (first || last) {
+      const T e = s[pg.s.e[ax] + f], head = first ? p : hi;  // Phi(1)
+      const T jmp = s[pg.s.j[ax] + f] + (head - e);
+      if (first) {
+        vlo = head - jmp;
+        slo = lo + (head - e);
+      }
+      if (last) {
+        vhi = head - jmp;
+        shi = e;
+      }
+    }
+    *nsum = slo + shi;
+    const T d = (T)di;
+    return di * ((double)pfma<T>(d, p - vhi, b) - (double)pfma<T>(d, lo - vlo, a));
+  };
+  for (int t = blockIdx.x * 256 + threadIdx.x; t < total; t += gridDim.x * 256) {
+    const int i = 1 + 2 * (t % hx), r = t / hx, j = 1 + r % ny, k = 1 + r / ny;
     const int o = pg.s.at(i, j, k);
     const int64_t c = g.at(i, j, k);
-    const T p = phi[o];
-    // of an axis: the divergence of the two faces as stored, and the sum of
-    // the two neighbours as the sweeps see them.  lo, hi: the neighbours'
-    // images; a, b: the low and the high face's velocity; (first, last): the
-    // cell lies there, f: its place on the face.
-    auto axis = [&](int ax, T lo, T hi, T a, T b, bool first, bool last, int f, double di, T* nsum) {
-      T vlo = p, vhi = hi;  // the high neighbour of the low face's cell, and of this one, as k_pot_apply has them
-      T slo = lo, shi = hi;
-      if (first || last) {
-        const T e = s[pg.s.e[ax] + f], head = first ? p : hi;  // Phi(1)
-        const T jmp = s[pg.s.j[ax] + f] + (head - e);
-        if (first) {
-          vlo = head - jmp;
-          slo = lo + (head - e);
-        }
-        if (last) {
-          vhi = head - jmp;
-          shi = e;
-        }
-      }
-      *nsum = slo + shi;
-      const T d = (T)di;
-      return di * ((double)pfma<T>(d, p - vhi, b) - (double)pfma<T>(d, lo - vlo, a));
-    };
-    const bool x1 = i == 1, xn = i == nx, y1 = j == 1, yn = j == ny, z1 = k == 1, zn = k == nz;
+    const bool x1 = i == 1, xn = i + 1 == nx, y1 = j == 1, yn = j == ny, z1 = k == 1, zn = k == nz;
+    const pair_t<T> p = lds2(phi + o), u = lds2(U + c), v = lds2(V + c), w = lds2(W + c);
+    const T pw = phi[x1 ? o + (nx - 1) : o - 1], pe = phi[xn ? o - (nx - 2) : o + 2], uw = U[x1 ? c + (nx - 1) : c - 1];
+    const pair_t<T> ps = lds2(phi + (y1 ? o + (ny - 1) * px : o - px)), pn = lds2(phi + (yn ? o - (ny - 1) * px : o + px));
+    const pair_t<T> pb = lds2(phi + (z1 ? o + (nz - 1) * pz : o - pz)), pt = lds2(phi + (zn ? o - (nz - 1) * pz : o + pz));
+    const pair_t<T> vs = lds2(V + (y1 ? g.at(i, ny, k) : c - g.px)), wb = lds2(W + (z1 ? g.at(i, j, nz) : c - g.pz));
+    pair_t<T> d = lds2(D + o);  // (without the x jumps so far)
     const int fx = (k - 1) * ny + (j - 1), fy = (k - 1) * nx + (i - 1), fz = (j - 1) * nx + (i - 1);
+    if (x1) d.x -= cx * s[pg.s.j[0] + fx];
+    if (xn) d.y += cx * s[pg.s.j[0] + fx];
     T sx, sy, sz;
-    double div = axis(0, phi[x1 ? o + (nx - 1) : o - 1], phi[xn ? o - (nx - 1) : o + 1],
-                      U[x1 ? c + (nx - 1) : c - 1], U[c], x1, xn, fx, pg.dxi, &sx);
-    div += axis(1, phi[y1 ? o + (ny - 1) * px : o - px], phi[yn ? o - (ny - 1) * px : o + px],
-                V[y1 ? g.at(i, ny, k) : c - g.px], V[c], y1, yn, fy, pg.dyi, &sy);
-    div += axis(2, phi[z1 ? o + (nz - 1) * pz : o - pz], phi[zn ? o - (nz - 1) * pz : o + pz],
-                W[z1 ? g.at(i, j, nz) : c - g.pz], W[c], z1, zn, fz, pg.dzi, &sz);
-    T d = D[o];  // (without the x jumps so far)
-    if (x1) d -= cx * s[pg.s.j[0] + fx];
-    if (xn) d += cx * s[pg.s.j[0] + fx];
-    const double e = div - (double)pot_div<T>(p, sx, sy, sz, d, cx, cy, cz);
-    acc += e * e;
+    double div = axis(0, p.x, pw, p.y, uw, u.x, x1, false, fx, pg.dxi, &sx);
+    div += axis(1, p.x, ps.x, pn.x, vs.x, v.x, y1, yn, fy, pg.dyi, &sy);
+    div += axis(2, p.x, pb.x, pt.x, wb.x, w.x, z1, zn, fz, pg.dzi, &sz);
+    const double ea = div - (double)pot_div<T>(p.x, sx, sy, sz, d.x, cx, cy, cz);
+    div = axis(0, p.y, p.x, pe, u.x, u.y, false, xn, fx, pg.dxi, &sx);
+    div += axis(1, p.y, ps.y, pn.y, vs.y, v.y, y1, yn, fy + 1, pg.dyi, &sy);
+    div += axis(2, p.y, pb.y, pt.y, wb.y, w.y, z1, zn, fz + 1, pg.dzi, &sz);
+    const double eb = div - (double)pot_div<T>(p.y, sx, sy, sz, d.y, cx, cy, cz);
+    acc += ea * ea + eb * eb;
   }
   return acc;
 }
 
 // FP32, after a couple that ran to its last sweep: the rounding of the stored
 // velocity into the residual that the log shows (a couple that left by the exit
-// test has it: k_pot_jump).  12 us at 32^3, 240 at 256^3, 1.8 ms at 512^3.
+// test has it: k_pot_jump).  12 us at 32^3, 71 at 192^3, 0.92 ms at 512^3
+// (a cell a thread 1.8).
 template <typename T>
 __global__ void __launch_bounds__(256) k_pot_round(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg,
                                                    HsmacCoef cf) {
@@ -239,15 +244,17 @@ __global__ void __launch_bounds__(256) k_pot_round(const __grid_constant__ PotGr
 // So when a sweep's own residual would let the couple end, its group's tests
 // wait (pot_check = 1): this kernel, the first of the next group, measures the
 // rounding at the group's output (pot_round_sum) and its last block runs the
-// tests, and that group does nothing else (pot_check = 2 until its sweep ends).
-// A measurement holds for the groups after it while it keeps the residual above
+// tests; that group's other kernels do nothing (cs.cont = 2 until the next one).
+// A measurement holds for the sweeps after it while it keeps the residual above
 // the exit by a factor of two in the square, for at most kPotRoundAge of them
 // (a couple at 32^3 passes an exit of 1e-8 after 250 sweeps and goes on to 300:
 // two measurements, 20 us each; after every eighth group they took 8 % of a step).
-constexpr int kPotRoundAge = 32;
+// Its registers are bounded for the jumps' sake (512^3: FP32 23 us with 64, 34
+// with 96; FP64 22 us with 32, 26 with 62).
+constexpr int kPotRoundAge = 96;
 template <typename T>
-__global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg,
-                                                  HsmacCoef cf) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 7)
+    k_pot_jump(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg, HsmacCoef cf, PotLoop loop) {
   const int m = blockIdx.y;
   Ctx* ctx = ga.ctx[m];
   const int done = ctx->cs.done, cont = ctx->cs.cont, pending = ctx->pot_pending, check = ctx->pot_check;  // one latency
@@ -264,11 +271,14 @@ __global__ void __launch_bounds__(256) k_pot_jump(const __grid_constant__ PotGro
       if (threadIdx.x != 0) return;
       ctx->ticket = 0;
       ctx->pot_round = sum * (cf.count / ((double)pg.s.nx * pg.s.ny * pg.s.nz));
-      ctx->pot_age = 0;
+      ctx->pot_since = ctx->cs.itr;
+      ctx->pot_check = 0;
       pot_exit(ctx, cf, ctx->pot_sum, ctx->pot_round);
-      ctx->pot_check = 2;
+      if (ctx->cs.cont) ctx->cs.cont = 2;
+      if (loop.on) cudaGraphSetConditional(loop.handle, couple_goes_on(ctx, loop.max_groups) ? 1u : 0u);
       return;
     }
+    if (cont == 2 && blockIdx.x == 0 && threadIdx.x == 0) ctx->cs.cont = 1;  // (2 or 1: the other blocks go on alike)
   }
   if (!pending) return;
   const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz;
@@ -497,8 +507,8 @@ __global__ void __launch_bounds__(kPotSlabThreads) k_pot_slab(const __grid_const
   const int m = blockIdx.y, b = blockIdx.x;
   const Ctx* ctx = ga.ctx[m];
   // (a group that runs again finds these in place)
-  const int done = ctx->cs.done, cont = ctx->cs.cont, redo = ctx->pot_redo, check = ctx->pot_check;
-  if (done || !cont || redo || check) return;
+  const int done = ctx->cs.done, cont = ctx->cs.cont, redo = ctx->pot_redo;
+  if (done || cont != 1 || redo) return;
   T* sh = (T*)pot_smem;  // [10][32][32]
   if (b < pg.slab0[1]) pot_slab_body<T, 2>(ga, pg, m, b, sh, red);
   else if (b < pg.slab0[0]) pot_slab_body<T, 1>(ga, pg, m, b - pg.slab0[1], sh, red);
@@ -554,18 +564,8 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   int* sZ = (int*)((T*)pot_smem + L::d_elems + L::x_elems);  // box bits of the planes kb - 13 ..
   const int m = blockIdx.y;
   Ctx* ctx = ga.ctx[m];
-  const int done = ctx->cs.done, cont = ctx->cs.cont, cur = ctx->pot_cur, redo = ctx->pot_redo, check = ctx->pot_check;
-  if constexpr (sizeof(T) == 4) {
-    if (check) {  // this group ran the last one's exit tests (k_pot_jump); they may have ended the couple
-      if (last_block(&ctx->ticket, gridDim.x, &last_flag) && threadIdx.x == 0) {
-        ctx->ticket = 0;
-        ctx->pot_check = 0;
-        if (loop.on) cudaGraphSetConditional(loop.handle, couple_goes_on(ctx, loop.max_groups) ? 1u : 0u);
-      }
-      return;
-    }
-  }
-  if (done || !cont) return;
+  const int done = ctx->cs.done, cont = ctx->cs.cont, cur = ctx->pot_cur, redo = ctx->pot_redo;
+  if (done || cont != 1) return;
   const int nsw = redo ? redo : 3;  // sweeps of this pass
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int nx = pg.s.nx, ny = pg.s.ny, nz = pg.s.nz;
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   }
   if (!last_block(&ctx->ticket, nb, &last_flag)) return;
   const double round = sizeof(T) == 4 ? ctx->pot_round : 0.0;
-  const int itr = ctx->cs.itr, age = ctx->pot_age + 1;
+  const int itr = ctx->cs.itr, since = ctx->pot_since;
   double sum[3];
 #pragma unroll
   for (int q = 0; q < 3; q++) {
@@ -829,14 +829,11 @@ __global__ void __launch_bounds__(PotTile<T, NW, RW>::NT, 1)
   } else {
     bool wait = false;
     if constexpr (sizeof(T) == 4) {
-      for (int q = 0; q < 3; q++)
-        if (itr + q >= cf.itrmin &&
-            (sum[q] + 0.5 * round <= pg.exit_sum || (sum[q] <= pg.exit_sum && age >= kPotRoundAge)))
-          wait = true;
-      wait = wait && isfinite(sum[0] + sum[1] + sum[2]);
+      const double least = fmin(sum[0], fmin(sum[1], sum[2]));
+      wait = least <= pg.exit_sum && itr + 2 >= cf.itrmin && isfinite(sum[0] + sum[1] + sum[2]) &&
+             (least + 0.5 * round <= pg.exit_sum || itr >= since + kPotRoundAge);
       if (wait || itr + 3 >= cf.itrmax)  // (k_pot_jump or k_pot_round adds the rounding to them)
         for (int q = 0; q < 3; q++) ctx->pot_sum[q] = sum[q];
-      if (round > 0.0) ctx->pot_age = age;
     }
     if (wait) ctx->pot_check = 1;
     else pot_exit(ctx, cf, sum, round);

@@ -114,7 +114,7 @@ constexpr size_t kPotSlabPlanes = 10;  // of 32 x 32 values in a slab block's sh
 template <typename T>
 struct PotKernels {
   void (*setup)(PotGroup<T>, Grid, int, PotGeom);
-  void (*jump)(PotGroup<T>, Grid, int, PotGeom, HsmacCoef);
+  void (*jump)(PotGroup<T>, Grid, int, PotGeom, HsmacCoef, PotLoop);
   void (*slab)(PotGroup<T>, PotGeom);
   void (*sweep[3])(PotGroup<T>, PotGeom, HsmacCoef, PotLoop);  // Tall, Mid, Flat
   void (*round)(PotGroup<T>, Grid, int, PotGeom, HsmacCoef);   // FP32 only
