@@ -321,21 +321,29 @@ class Engine : public EngineBase {
   // ------------------------------------------------------- potential form
   // The time-blocked couple in potential form (lcs_potential.cuh) serves
   // red-black-fast.  LCS_B200_FUSED_SWEEP = rw or plain, or a variable that
-  // shapes those sweeps (LCS_B200_RW, _FACES, _ZCHUNK), selects the
-  // element-wise sweeps, and so does the test hook of their device waits.
-  // FP64 grids of up to 40^3 cells keep them too: there they give the in-place
-  // order's bits, and a step is a few milliseconds either way.
+  // shapes those sweeps (LCS_B200_RW, _FACES, _ZCHUNK; not beside
+  // LCS_B200_FUSED_SWEEP = potential), selects the element-wise sweeps, and so
+  // does the test hook of their device waits.
+  //
+  // FP64 grids of up to 40^3 cells keep the element-wise sweeps, for their bits
+  // and not for speed: a step of such a box equals the reference's in-place
+  // order bit for bit, which is what its results are compared by, and the
+  // potential form equals it to 1e-14.  It would be twice as fast there too (ms
+  // a step, element-wise and potential: 16^3 1.98 and 1.01, 24^3 3.68 and 1.81,
+  // 32^3 6.75 and 3.41, 40^3 11.8 and 5.3; above the line 48^3 18.2 and 8.3), and
+  // LCS_B200_FUSED_SWEEP = potential selects it.
   bool pot_ok = false;
   int debug_kind = 0;
   int pot_tile = -1;  // LCS_B200_POT_TILE = 0, 1 or 2 (tests and timing): that tile of the sweep
   bool use_pot() const { return pot_ok && debug_kind == 0; }
-    // Tiles of the sweep (warps x rows a warp).  Taller tiles do less redundant
+  // Tiles of the sweep (warps x rows a warp).  Taller tiles do less redundant
   // work, a plane of shorter ones takes less time, and a grid of few tiles
   // leaves SMs idle that shorter ones would use; pot_geom weighs them by the
   // time of a plane.  Measured, us a launch with tiles of 36, 20 and 4 rows
-  // (FP64: 20 and 4): FP32 32^3 33, 27, 21; 48^3 33, 27, 24; 64^3 35, 31, 35;
-  // 96^3 43, 37, 64; 128^3 60, 56, 122; 192^3 117, 127, 273; 256^3 240, 228;
-  // 512^3 1044, 1199.  FP64 48^3 33, 29; 64^3 40, 41; 96^3 52, 77.
+  // (FP64: 20 and 4): FP32 32^3 33, 27, 23; 48^3 34, 29, 25; 64^3 35, 31, 36;
+  // 96^3 45, 37, 66; 128^3 60, 58, 128; 192^3 117, 130, 283; 256^3 254, 232;
+  // 384^3 590, 646; 512^3 1102, 1252.  FP64 48^3 35, 29; 64^3 40, 42; 96^3 51, 78;
+  // 128^3 82, 154.
   using PotT = typename PotTiles<T>::Tall;
   using PotS = typename PotTiles<T>::Mid;
   using PotV = typename PotTiles<T>::Flat;
@@ -441,10 +449,7 @@ class Engine : public EngineBase {
     const int M = pot_members();
     if (3 * (int64_t)pg.nseg + pg.nslab > plan.partials_cap) return fail(LCS_EINVAL, "grid too large for the partials buffer");
     const int64_t faces = (int64_t)g.n[0] * g.n[1] + (int64_t)g.n[0] * g.n[2] + (int64_t)g.n[1] * g.n[2];
-    // (FP32: it has all cells to visit when it measures the velocity's rounding)
-    const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2], jump = sizeof(T) == 4 ? std::max(faces, cells / 4) : faces;
-    LCS_TRY(launch("pot_jump", pot.jump, dim3(blocks_for(jump, 256), M), dim3(256), 0, pot_args(), g, set, pg, hc,
-                   loop));
+    LCS_TRY(launch("pot_jump", pot.jump, dim3(blocks_for(faces, 256), M), dim3(256), 0, pot_args(), g, set, pg, hc, loop));
     if (cfg.overlap)
       LCS_TRY(launch("pot_slab", pot.slab, dim3(pg.nslab, M), dim3(kPotSlabThreads), kSlabSmem, pot_args(), pg));
     const dim3 grid(pg.nseg, M);
