@@ -58,8 +58,9 @@ OTHER_WORKLOADS = ("batch64", "serve", "makeindex", "couple256")
 # reports them.
 SWEEP_DRAM_BYTES_PER_CELL = {"fp64": 67.8, "fp32-mixed": 35.5}
 SWEEP_KERNELS = ("pot_sweep", "hsmac_rw", "hsmac_fused")
-# the same of pot_sweep, which does three sweeps a launch (512^3 captures)
-POT_DRAM_BYTES_PER_CELL = {"fp64": 39.0, "fp32-mixed": 18.6}
+# the same of pot_sweep, which does three sweeps a launch (captures at 512^3,
+# profiles/pot_sweep.md)
+POT_DRAM_BYTES_PER_CELL = {"fp64": 39.0, "fp32-mixed": 18.4}
 # FP64 operations per interior cell of one rhs!+update! launch (k_rhs, both
 # stages alike): smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on
 # of an ncu capture of k_rhs at 128^3: 484.4 M adds + 471.9 M multiplies, no
@@ -676,7 +677,8 @@ def kernel_bytes(n, h, T, particles_per_launch):
     h, T-byte field elements):
     - pot_sweep: Phi and its right-hand side read, Phi written, 3T x n^3 (three
       sweeps); pot_setup: U, V, W read, the two written, 5T; pot_apply: Phi, U,
-      V, W, P read, the last four written, 9T;
+      V, W, P read, the last four written, 9T; pot_round (FP32): Phi, its
+      right-hand side, U, V, W read, 5T;
     - hsmac_rw: U, V, W, P read and written once per cell, 8T x n^3;
     - hsmac_faces: the same per cell of the six face slabs of the first
       time-blocked sweep's box -1..n+3 around the core 2..n;
@@ -690,7 +692,8 @@ def kernel_bytes(n, h, T, particles_per_launch):
     n3 = float(n) ** 3
     slab = float(n + 5) ** 3 - float(n - 1) ** 3
     halo = float(n + 2 * h) ** 3 - n3
-    return {"pot_sweep": 3 * T * n3, "pot_setup": 5 * T * n3, "pot_apply": 9 * T * n3, "hsmac_rw": 8 * T * n3, "hsmac_faces": 8 * T * slab, "synchalo": 3 * 2 * T * halo,
+    return {"pot_sweep": 3 * T * n3, "pot_setup": 5 * T * n3, "pot_apply": 9 * T * n3, "pot_round": 5 * T * n3,
+            "hsmac_rw": 8 * T * n3, "hsmac_faces": 8 * T * slab, "synchalo": 3 * 2 * T * halo,
             "rhs_update": 8.5 * T * n3, "particles": 128.0 * particles_per_launch, "cfl_max": 3 * T * n3}
 
 

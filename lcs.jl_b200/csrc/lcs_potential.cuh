@@ -72,7 +72,7 @@ __device__ __forceinline__ int pot_layer(int i, int nx) { return i <= 4 ? 2 + i 
 __device__ __forceinline__ int pot_dlayer(int i, int nx) { return i <= 3 ? 1 + i : i >= nx - 1 ? i - (nx - 1) : -1; }
 
 // Start of a couple: D = div U (periodic, in FP64, rounded once), Phi = 0, J = 0.
-// Bound by HBM: 3 fields read, 2 written (512^3: FP64 1.2 ms, 4.5 TB/s).
+// Bound by HBM: 3 fields read, 2 written (512^3: FP64 1.2 ms, FP32 0.75).
 template <typename T>
 __global__ void __launch_bounds__(256) k_pot_setup(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg) {
   const int m = blockIdx.y;
@@ -356,11 +356,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 7)
 // of the core, then of the z slabs, the y slabs and the x slabs, as far as the
 // block's columns and its axis need them.  Blocks at the rim of a y or x slab
 // so sweep the few cells of the earlier slabs beside it themselves, and no
-// block waits for another: one launch instead of three (a step at 96^3 in FP32
-// 13.4 -> 10.4 ms, 512^3 as before).  Bound by the latency of its loads and its
-// four to eight phases (11 us up to 128^3).  A value reaches at most 5 columns (both colours of the
-// x, the y and the z slab, where the y slab crosses to the z slab in place),
-// so 22 x 22 of the columns are the block's own.
+// block waits for another: one launch for the three axes.  A cell that two
+// blocks sweep is stored by one of them; the other's may differ from it in the last bits, since a block sums the
+// axes in its own order and an x block's D has its jumps added one by one.
+// Bound by the latency of its loads and its four to eight phases (17 to 19 us up
+// to 128^3, 98 and 112 at 512^3 in FP32 and FP64).  A value reaches at most 5
+// columns (both colours of the x, the y and the z slab, where the y slab crosses
+// to the z slab in place), so 22 x 22 of the columns are the block's own.
 template <typename T, int AX>
 __device__ __forceinline__ void pot_slab_body(const PotGroup<T>& ga, const PotGeom& pg, int m, int tile, T* sh,
                                               double* red) {
@@ -542,11 +544,12 @@ __device__ __forceinline__ double pot_keep(double v, int mask) {
 // the outer layers; without, the halo is the periodic image, read in place
 // (pairs never straddle the period: n is even).
 //
-// A group at 512^3: FP32 1.05 ms (12 x 4 rows), FP64 1.8 ms (8 x 4), where the
-// three element-wise sweeps with their slabs and fill took 3.7 and 6.2; at the
+// A launch at 512^3: FP32 1.10 ms (12 x 4 rows), FP64 1.86 ms (8 x 4), where the
+// three element-wise sweeps with their slabs and fill take 3.7 and 6.2; at the
 // HBM peak its 3 values a cell take 0.25 and 0.49.  It is bound by instruction
-// issue and latency: issue 54 % (FP32) and 37 % (FP64) of the cycles, DRAM 29
-// and 35 %, the shared-memory pipe 41 and 53 %.  The tile is as tall as the
+// issue and latency (FP32 at 384^3, FP64 at 256^3): issue 47 and 27 % of the
+// cycles (63 and 44 % of those of an SM that has a CTA), DRAM 19 and 16 %, the
+// shared-memory pipe 44 and 54 %.  The tile is as tall as the
 // registers allow (168 and 254 a thread): a row's two colours at 7 planes live
 // in them, and D, read once in three half sweeps each, in shared memory.
 template <typename T, int NW, int RW>
