@@ -247,11 +247,11 @@ __global__ void __launch_bounds__(256) k_pot_round(const __grid_constant__ PotGr
 // tests; that group's other kernels do nothing (cs.cont = 2 until the next one).
 // A measurement holds for the sweeps after it while it keeps the residual above
 // the exit by a factor of two in the square, for at most kPotRoundAge of them
-// (a couple at 32^3 passes an exit of 1e-8 after 250 sweeps and goes on to 300:
-// two measurements, 20 us each; after every eighth group they took 8 % of a step).
+// (a couple at 32^3 passes an exit of 1e-8 after about 180 sweeps and goes on to
+// 300: one measurement, 25 us; every 24 sweeps they took 8 % of a step).
 // Its registers are bounded for the jumps' sake (512^3: FP32 23 us with 64, 34
 // with 96; FP64 22 us with 32, 26 with 62).
-constexpr int kPotRoundAge = 96;
+constexpr int kPotRoundAge = 256;
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 7)
     k_pot_jump(const __grid_constant__ PotGroup<T> ga, Grid g, int set, PotGeom pg, HsmacCoef cf, PotLoop loop) {
@@ -357,12 +357,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 7)
 // block's columns and its axis need them.  Blocks at the rim of a y or x slab
 // so sweep the few cells of the earlier slabs beside it themselves, and no
 // block waits for another: one launch for the three axes.  A cell that two
-// blocks sweep is stored by one of them; the other's may differ from it in the last bits, since a block sums the
-// axes in its own order and an x block's D has its jumps added one by one.
-// Bound by the latency of its loads and its four to eight phases (17 to 19 us up
-// to 128^3, 98 and 112 at 512^3 in FP32 and FP64).  A value reaches at most 5
-// columns (both colours of the x, the y and the z slab, where the y slab crosses
-// to the z slab in place), so 22 x 22 of the columns are the block's own.
+// blocks sweep is stored by one of them; the other's may differ from it in the
+// last bits, since a block sums the axes in its own order and an x block's D has
+// its jumps added one by one.  Bound by the latency of its loads and its four to
+// eight phases (17 to 19 us up to 128^3, 98 and 112 at 512^3 in FP32 and FP64).
+// A value reaches at most 5 columns (both colours of the x, the y and the z slab,
+// where the y slab crosses to the z slab in place), so 22 x 22 of the columns are
+// the block's own.
 template <typename T, int AX>
 __device__ __forceinline__ void pot_slab_body(const PotGroup<T>& ga, const PotGeom& pg, int m, int tile, T* sh,
                                               double* red) {
